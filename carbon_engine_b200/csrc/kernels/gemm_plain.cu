@@ -1,5 +1,5 @@
-// y = x * W^T with float32 FMA arithmetic: the matrix product of the float32 path, and the plain
-// twin (and odd-size fallback) of the tensor-core products.
+// y = x * W^T with float32 FMA arithmetic on bfloat16 operands: the plain twin (and odd-size fallback) of the tensor-core
+// products.  (Float32 operands go to gemm_f32.cu.)
 //
 // x is [M, K], W is [N, K] (a linear layer's weight as stored, src/model/layers.rs:441), both
 // row-major.  Every output element is one thread's running sum over k = 0, 1, 2, ... in that order,
@@ -10,18 +10,11 @@
 // SwiGLU, where W holds the gate rows [0, N) and the up rows [N, 2N) and the output is
 // silu(gate) * up (src/model/layers.rs:625-648), relu(gate) * up, or the clamped gated activation of gate and up rows
 // with an optional bias.
-#include "common.cuh"
+#include "gemm_f32.cuh"
 
 #define GP_BM 64
 #define GP_BN 64
 #define GP_BK 16
-
-enum { GP_STORE = 0, GP_STORE_F32 = 1, GP_ACCUM_F32 = 2, GP_SWIGLU = 3, GP_RELUGLU = 4, GP_RELU2 = 5, GP_CLAMPGLU = 6 };     // 4: relu(gate) * up; 5: relu(v)^2; 6: ce_clamp_glu(gate + bias, up + bias)
-
-struct GpGate {
-    const float* bias;           // float32 [2N] or null: gate rows, then up rows (mode 6)
-    float limit, alpha;
-};
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256) gemm_plain_kernel(const T* __restrict__ A, const T* __restrict__ W,
@@ -127,7 +120,8 @@ extern "C" int ce_gemm_plain(const void* A, const void* W, void* C, int dtype, i
     if (!A || !W || !C) return ce_fail(CE_ERR_ARG, "ce_gemm_plain: null pointer");
     if (K <= 0) return ce_fail(CE_ERR_SIZE, "ce_gemm_plain: K=%d", K);
     if ((M + GP_BM - 1) / GP_BM > 65535) return ce_fail(CE_ERR_SIZE, "ce_gemm_plain: M=%d is too large", M);
-    if (dtype == CE_F32) return launch_plain<float>(A, W, C, M, N, K, lda, ldc, mode, gate, stream);
+    if (mode < GP_STORE || mode > GP_CLAMPGLU) return ce_fail(CE_ERR_ARG, "ce_gemm_plain: unknown epilogue %d", mode);
+    if (dtype == CE_F32) return ce_gemm_f32((const float*)A, (const float*)W, (float*)C, M, N, K, lda, ldc, mode, gate, stream);
     if (dtype == CE_BF16) return launch_plain<__nv_bfloat16>(A, W, C, M, N, K, lda, ldc, mode, gate, stream);
     return ce_fail(CE_ERR_ARG, "ce_gemm_plain: unknown dtype %d", dtype);
 }

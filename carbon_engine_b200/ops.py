@@ -700,7 +700,7 @@ def attention_generic(q, q_stride: int, k_pool, v_pool, out, positions, seq_of_t
 
 
 def gemm_plain(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, mode: int, glu: Optional[GluParams] = None) -> None:
-    """c = a @ w.T with float32 FMA arithmetic; see csrc/kernels/gemm_plain.cu for the epilogues."""
+    """c = a @ w.T with float32 FMA arithmetic; see csrc/kernels/gemm_f32.cuh for the epilogues."""
     _need(w, "w", a.dtype); _need(c, "c")
     if a.stride(-1) != 1 or c.stride(-1) != 1:
         raise KernelError("gemm_plain: rows must be contiguous")
