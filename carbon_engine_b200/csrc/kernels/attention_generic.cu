@@ -1,5 +1,5 @@
 // Causal grouped-query attention over the paged cache, for any number of new tokens per sequence,
-// in plain float32 arithmetic.  It is the attention of the float32 path and the plain twin of the
+// in plain float32 arithmetic.  It is the float32 path's where attention_f32.cu refuses the sizes, and the plain twin of the
 // tensor-core kernels.
 //
 // One block per (token, query head).  The query at absolute position p sees keys lo..p, where

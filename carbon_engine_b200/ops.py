@@ -699,6 +699,21 @@ def attention_generic(q, q_stride: int, k_pool, v_pool, out, positions, seq_of_t
         k_pool.shape[0], int(window), float(scale), _stream()))
 
 
+def attention_f32(q, q_stride: int, k_pool, v_pool, out, positions, seq_slot, q_start, block_table, tiles, status, n_decode: int,
+                  n_tiles: int, nh: int, nkv: int, d: int, page_size: int, window: int, max_ctx: int, scale: float) -> bool:
+    """Float32 attention of a step: its first ``n_decode`` sequences bring one token each, ``tiles`` ((sequence, first token) pairs)
+    cover the others 64 tokens at a time; ``max_ctx``: the longest sequence's keys.  False if the sizes or layouts are not the kernel's (:func:`attention_generic` takes them)."""
+    if any(t.dtype != torch.float32 for t in (q, k_pool, v_pool, out)) or not kernels().ce_attention_f32_supported(nh, nkv, d, q_stride) or \
+            (q.data_ptr() | k_pool.data_ptr() | v_pool.data_ptr() | out.data_ptr()) & 15:
+        return False
+    _need(k_pool, "k_pool"); _need(v_pool, "v_pool"); _need(out, "out")
+    _ok(kernels().ce_attention_f32(
+        _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(out), _ptr(positions), _ptr(seq_slot), _ptr(q_start), _ptr(block_table), _ptr(tiles),
+        _ptr(status), n_decode, n_tiles, nh, nkv, d, q_stride, page_size, block_table.shape[1], k_pool.shape[0], int(window),
+        int(max_ctx), float(scale), _stream()), (n_decode > 0) + (n_tiles > 0))
+    return True
+
+
 def gemm_plain(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, mode: int, glu: Optional[GluParams] = None) -> None:
     """c = a @ w.T with float32 FMA arithmetic; see csrc/kernels/gemm_f32.cuh for the epilogues."""
     _need(w, "w", a.dtype); _need(c, "c")

@@ -153,5 +153,10 @@ class PagedAttention(Mixer):
             if ops_tensor.attention_bf16(ctx, ctx.plans[self.plan_key], qkv, out, cache, table, nh, nkv, d, self.window,
                                          self.scale):
                 return
+        plan = ctx.plans[self.plan_key]
+        if qkv.dtype == torch.float32 and ops.attention_f32(
+                qkv, qkv.shape[1], cache.k_pool, cache.v_pool, out, ctx.positions, ctx.seq_slot, ctx.q_start, table, plan.tiles,
+                ctx.status, ctx.n_decode, plan.n_tiles, nh, nkv, d, cache.page_size, self.window, ctx.max_ctx, self.scale):
+            return
         ops.attention_generic(qkv, qkv.shape[1], cache.k_pool, cache.v_pool, out, ctx.positions, ctx.seq_of_token,
                               ctx.seq_slot, table, ctx.status, nh, nkv, d, cache.page_size, self.window, self.scale)

@@ -1,11 +1,12 @@
-"""The float32 path's product at the edges of its tiles and runs, against float64, and bit for bit over the
+"""The float32 path's product and attention at the edges of their tiles, runs and chunks, against float64, and bit for bit over the
 ways a step can be cut."""
 import math
 
 import pytest
 import torch
 
-from test_kernels_gpu import dev
+import plain_qwen3 as plain
+from test_kernels_gpu import dev, fill_pools, paged_layout, status, step_meta
 
 pytestmark = pytest.mark.gpu
 
@@ -58,3 +59,69 @@ def test_float32_product_has_the_same_bits_in_every_tile_and_cluster(N, K):
     whole = product(a, w, ops.GEMM_STORE)
     for lo, n in ((0, 1), (3, 4), (1, 7), (30, 33), (2, 64), (5, 65)):
         assert torch.equal(product(a[lo:lo + n], w, ops.GEMM_STORE), whole[lo:lo + n]), n
+
+
+def attention(seqs, q, kp, vp, table, nh, nkv, d, ps, window, stride):
+    from carbon_engine_b200 import ops
+    T = sum(n for _, n in seqs)
+    positions, _, slots = step_meta(seqs)
+    starts = [0]
+    for _, n in seqs:
+        starts.append(starts[-1] + n)
+    n_decode = next((b for b, (_, n) in enumerate(seqs) if n > 1), len(seqs))
+    tiles = [(b, t) for b, (_, n) in enumerate(seqs) if b >= n_decode for t in range(0, n, 64)]
+    ints = lambda x: torch.tensor(x, dtype=torch.int32, device=dev())
+    out, st = torch.full((T, nh * d), 7.0, device=dev()), status()
+    assert ops.attention_f32(q, stride, kp, vp, out, positions, slots, ints(starts), table, ints(tiles or [(0, 0)]), st, n_decode, len(tiles),
+                             nh, nkv, d, ps, window, max(c + n for c, n in seqs), 1 / math.sqrt(d))
+    return out, int(st.item())
+
+
+# groups of 1, 2, 3, 8, 9 and 20 heads; head sizes below, at and above a column round; pages smaller and larger than a chunk; windows
+# that start inside a chunk
+@pytest.mark.parametrize("nh,nkv,d,ps,window", [(2, 2, 16, 16, 0), (6, 3, 20, 5, 0), (3, 1, 64, 64, 0), (8, 1, 68, 8, 70), (18, 2, 128, 128, 0),
+                                                 (20, 1, 100, 7, 130)])
+def test_float32_attention_against_float64(nh, nkv, d, ps, window):
+    torch.manual_seed(2)
+    seqs = [(0, 1), (63, 1), (64, 1), (700, 1), (0, 2), (61, 7), (0, 64), (0, 65), (600, 130)]
+    table, kp, vp = paged_layout([c + n for c, n in seqs], ps, nkv, d, torch.float32, shuffle_seed=3)
+    T = sum(n for _, n in seqs)
+    stride = (nh + 2 * nkv) * d
+    q, want, t = torch.full((T, stride), float("nan"), device=dev()), [], 0
+    for b, (ctx, n) in enumerate(seqs):
+        q_all, k_all, v_all = torch.randn(ctx + n, nh, d) * 1.5, torch.randn(ctx + n, nkv, d) * 1.5, torch.randn(ctx + n, nkv, d)
+        fill_pools(kp, vp, table.cpu().numpy(), b, k_all.to(dev()), v_all.to(dev()), ps)
+        q[t:t + n, :nh * d] = q_all[ctx:].reshape(n, nh * d).to(dev())
+        want.append(plain.causal_attention(q_all.double(), k_all.double(), v_all.double(), 1 / math.sqrt(d), window)[ctx:])
+        t += n
+    out, st = attention(seqs, q, kp, vp, table, nh, nkv, d, ps, window, stride)
+    want = torch.cat(want)
+    # scores of size |q| |k| / sqrt(d) ~ 2 sqrt(d) carry d / 2 roundings each; their error is the probabilities' relative error
+    assert st == 0 and float((out.view(T, nh, d).double().cpu() - want).abs().max()) < 2e-5 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("nh,nkv,d,ps,window", [(16, 4, 128, 64, 0), (5, 1, 24, 16, 100)])
+def test_float32_attention_has_the_same_bits_however_the_step_is_cut(nh, nkv, d, ps, window):
+    """The last token's neighbours hold values no one before it may meet: a row of infinities at the last position."""
+    torch.manual_seed(3)
+    L = 777
+    table, kp, vp = paged_layout([L], ps, nkv, d, torch.float32, shuffle_seed=1)
+    k, v = torch.randn(L, nkv, d, device=dev()), torch.randn(L, nkv, d, device=dev())
+    v[L - 1] = float("inf")
+    fill_pools(kp, vp, table.cpu().numpy(), 0, k, v, ps)
+    q = torch.randn(L, nh * d, device=dev())
+    whole, st = attention([(0, L)], q, kp, vp, table, nh, nkv, d, ps, window, nh * d)
+    assert st == 0 and torch.isfinite(whole[:L - 1]).all()
+    for past, n in ((0, 5), (130, 500), (699, 1), (64, 1), (63, 2), (500, 277), (0, 1), (775, 1)):
+        got, st = attention([(past, n)], q[past:past + n].contiguous(), kp, vp, table, nh, nkv, d, ps, window, nh * d)
+        end = min(n, L - 1 - past)
+        assert st == 0 and torch.equal(got[:end], whole[past:past + end]), (past, n)
+
+
+def test_float32_attention_flags_a_page_the_request_does_not_hold():
+    table, kp, vp = paged_layout([200], 16, 1, 16, torch.float32)
+    fill_pools(kp, vp, table.cpu().numpy(), 0, torch.randn(200, 1, 16, device=dev()), torch.randn(200, 1, 16, device=dev()), 16)
+    table = table.clone()
+    table[0, 5] = -1
+    out, st = attention([(199, 1)], torch.randn(1, 16, device=dev()), kp, vp, table, 1, 1, 16, 16, 0, 16)
+    assert st == 4 and torch.isfinite(out).all()
