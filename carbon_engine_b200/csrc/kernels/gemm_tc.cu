@@ -26,6 +26,7 @@
 #include "common.cuh"
 #include "tensor_map.h"
 #include <mutex>
+#include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <unordered_map>
@@ -93,6 +94,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// One lane of a converged warp.  The MMA issuers' loops (and the pairs' producers') are walked by whole warps, and only the copies,
+// the MMAs and the commits are one lane's: operands that a converged warp computes stay in uniform registers, which is where those
+// instructions take them from; inside an `if (lane == 0)` every one of them is brought over first (pairs, 130 tokens, 4,096 features
+// of K = 12,288: 56 -> 48 us; 2,048 tokens, 12,288 gated features: 280 -> 268 us).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+    return p != 0;
 }
 
 // Optional timing trace (CE_GEMM_TRACE=1): block (0,0,0) of every launch stamps %globaltimer at a few
@@ -164,6 +175,19 @@ __device__ __forceinline__ void epilogue_store(const TcArgs& a, int m, int n, fl
     else if (a.mode == TC_ACCUM_F32) ((float*)a.out)[o] += v;
     else if (a.mode == TC_RELU2) { float r = fmaxf(v, 0.f); ((__nv_bfloat16*)a.out)[o] = __float2bfloat16_rn(r * r); }
     else ((__nv_bfloat16*)a.out)[o] = __float2bfloat16_rn(gated_mul<CLAMP>(a, v, up, CLAMP ? gate_bias(a, n, 0) : 0.f, CLAMP ? gate_bias(a, n, 1) : 0.f));
+}
+
+// The same without the gated activations, for epilogues that are unrolled over tokens: a block runs its epilogue once, so every
+// instruction of it is fetched from L2 first, and the activations' code, repeated for every token and never run, cost the store of
+// 130 x 4,096 results 6 us (two pairs a tile: 24 us, where adding into the residual took 18).
+__device__ __forceinline__ void store_plain(const TcArgs& a, int m, int n, float v) {
+    const size_t o = (size_t)m * a.ldo + n;
+    if (a.mode == TC_ACCUM_F32) ((float*)a.out)[o] += v;
+    else if (a.mode == TC_STORE_F32) ((float*)a.out)[o] = v;
+    else {
+        const float r = fmaxf(v, 0.f);
+        ((__nv_bfloat16*)a.out)[o] = __float2bfloat16_rn(a.mode == TC_RELU2 ? r * r : v);
+    }
 }
 
 template <int BN, int NACC, bool COOP, bool CLAMP = false>
@@ -364,7 +388,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_tc_kernel(const __grid_consta
                         } else {
 #pragma unroll
                             for (int j = 0; j < 16; ++j)
-                                if (c + j < m_valid) epilogue_store(a, m0 + c + j, n, g[j], 0.f);
+                                if (c + j < m_valid) store_plain(a, m0 + c + j, n, g[j]);
                         }
                     }
                 }
@@ -486,7 +510,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_tc_kernel(const __grid_consta
                         for (int j = 0; j < TB; ++j) {
                             if (mb + j >= m_hi) continue;
                             if (a.mode == TC_ACCUM_F32) ((float*)a.out)[(size_t)(m0 + mb + j) * a.ldo + n] = xv[j] + g[j];
-                            else epilogue_store(a, m0 + mb + j, n, g[j], 0.f);
+                            else store_plain(a, m0 + mb + j, n, g[j]);
                         }
                     }
                 }
@@ -533,7 +557,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_tc_kernel(const __grid_consta
                         float* xp = (float*)a.out + (size_t)(m0 + m) * a.ldo + n;
                         *xp = *xp + g;
                     } else {
-                        epilogue_store(a, m0 + m, n, g, 0.f);
+                        store_plain(a, m0 + m, n, g);
                     }
                 }
             }
@@ -862,7 +886,10 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_persistent_kernel(const __gri
                     } else {
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
-                            if (c + j < m_valid) epilogue_store<CLAMP>(a, m0 + c + j, n, g[j], NACC == 2 ? u[j] : 0.f);
+                            if (c + j < m_valid) {
+                                if (NACC == 2) epilogue_store<CLAMP>(a, m0 + c + j, n, g[j], u[j]);
+                                else store_plain(a, m0 + c + j, n, g[j]);
+                            }
                     }
                 }
             }
@@ -897,14 +924,14 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
 }
 __device__ __forceinline__ bool mbar_test_cluster(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+    asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
                  : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity) {
     for (uint32_t i = 0; i < SPIN_LIMIT; ++i) {
         uint32_t ok;
-        asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+        asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
                      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
         if (ok) return true;
         if (i > 64) __nanosleep(i > 4096 ? 1024 : 128);
@@ -921,42 +948,62 @@ __device__ __forceinline__ void umma2_bf16(uint32_t d_tmem, uint64_t a_desc, uin
     asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}"
                  ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void umma2_commit_both(uint64_t* bar) {
-    unsigned short mask = 3;          // the barrier at this offset in both CTAs of the pair
+__device__ __forceinline__ void umma2_commit_both(uint64_t* bar, uint32_t leader) {
+    unsigned short mask = (unsigned short)(3u << leader);          // the barrier at this offset in both CTAs of the pair
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                  ::"r"(smem_u32(bar)), "h"(mask) : "memory");
 }
 
-// BN: tokens per pair tile (each CTA loads BN/2 of them).  KSUB: k-blocks of 64 per stage (per barrier
+// A tile's tokens (btok, a multiple of 16; each CTA loads half of them) are the launch's choice: as many as split the step's tokens
+// evenly and fill whole waves of pairs.  KSUB: k-blocks of 64 per stage (per barrier
 // round of the MMA thread).  GU (SwiGLU): a CTA's 128 rows are 64 gate rows and the 64 up rows of the same
 // features, brought by two TMA boxes into ONE tile, so the product is the same single-accumulator product
 // as any other and a pair tile covers 128 features; in the epilogue the warps that hold the up rows (lanes
 // 64..127 of tensor memory) hand their values to the warps that hold the gate rows through shared memory.
-template <int BN, bool GU, int KSUB, bool CLAMP = false>
+//
+// SPLIT: a tile's rounds over K are dealt to the 2 to 4 pairs of a cluster, for products with too few tiles to give every pair one
+// (a few hundred tokens: 16 tiles of a 4,096-wide output for 74 pairs).  When all of the cluster's MMAs are done, the stages are
+// free, and every CTA writes the part of its accumulators that another pair is to finish into THAT CTA's shared memory; a pair
+// then adds the partial sums of its share of the tokens in split order and runs the epilogue for them.  The partial sums never
+// leave the SMs.
+constexpr int PAIR_MAX_TOKENS = 256;
+constexpr int PAIR_MAX_STAGES = 12;
+constexpr int PAIR_MAX_SPLITS = 4;               // four pairs are a cluster of eight, the portable limit
+// Wide tiles go through their stages one k-block at a time (more, smaller stages in flight), narrow ones two (half the barrier
+// rounds for MMAs that are half as long).  2,048 tokens, 12,288 gated features, tiles of 256: 268 us with two, 264 with one;
+// 130 tokens, 4,096 features of K = 12,288, tiles of 128: 48 us with two, 53 with one.
+__host__ __device__ constexpr int pair_ksub(int btok) { return btok >= 208 ? 1 : 2; }
+__host__ __device__ constexpr uint32_t pair_stage_bytes(int btok) { return pair_ksub(btok) * (BM * BK * 2 + (btok / 2) * BK * 2); }
+
+template <bool GU, int KSUB, bool CLAMP, bool SPLIT>
 __global__ void __launch_bounds__(THREADS) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w,
                                                               const __grid_constant__ CUtensorMap map_x, TcArgs a,
-                                                              int stages, int tiles_n, int tiles_m) {
+                                                              int stages, int tiles_n, int tiles_m, int btok) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t full_bar[8], empty_bar[8], acc_full[2], acc_empty[2];
+    __shared__ __align__(8) uint64_t full_bar[PAIR_MAX_STAGES], empty_bar[PAIR_MAX_STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int s_acc_ok;                         // the epilogue's verdict on a wait, taken by one thread for all 128
     __shared__ float xbuf[GU ? 2 * 2 * 64 * 17 : 1]; // GU: per buffer, 16 gate and 16 up values of 64 features (padded rows)
 
-    constexpr int HALF_N = BN / 2;
     constexpr int ROWS_N = GU ? BM / 2 : BM;         // output features of one CTA's tile
-    constexpr uint32_t W_BYTES = BM * BK * 2, X_BYTES = HALF_N * BK * 2;
-    constexpr uint32_t SUB_BYTES = W_BYTES + X_BYTES;                 // one k-block: weight rows, then tokens
-    constexpr uint32_t STAGE_BYTES = KSUB * SUB_BYTES;
-    constexpr uint32_t ACC_COLS = BN;
-    constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;
-    static_assert(TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0, "two accumulator sets must fit tensor memory");
-    const int rounds = (a.kblocks + KSUB - 1) / KSUB;                 // a k-block beyond K reads zeros
+    constexpr uint32_t W_BYTES = BM * BK * 2;
+    constexpr uint32_t ACC_COLS = PAIR_MAX_TOKENS;
+    constexpr uint32_t TMEM_COLS = SPLIT ? ACC_COLS : 2 * ACC_COLS;
+    const int half_n = btok / 2;
+    const uint32_t sub_bytes = W_BYTES + half_n * BK * 2;             // one k-block: weight rows, then tokens
+    const uint32_t stage_bytes = KSUB * sub_bytes;
+    const int all_rounds = (a.kblocks + KSUB - 1) / KSUB;             // a k-block beyond K reads zeros
     uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char* tiles = smem_raw + (base - smem_u32(smem_raw));
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t rank = cluster_rank();                  // 0: leader
-    int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-    int total = tiles_n * tiles_m;                   // pair tiles: tiles_n of 2 * ROWS_N features, tiles_m of BN tokens
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const uint32_t leader = cluster_rank() & ~1u;    // the pair's first CTA
+    const uint32_t rank = cluster_rank() & 1u;
+    const int part = SPLIT ? (int)(cluster_rank() >> 1) : 0;          // which part of K (and, in the end, of the tokens) is this pair's
+    const int group = SPLIT ? 2 * a.splits : 2;
+    int pair = blockIdx.x / group, n_pairs = gridDim.x / group;       // (SPLIT: the cluster's tile; there are as many clusters as tiles)
+    int total = tiles_n * tiles_m;                   // pair tiles: tiles_n of 2 * ROWS_N features, tiles_m of btok tokens
+    const int round0 = SPLIT ? all_rounds * part / a.splits : 0;
+    const int rounds = (SPLIT ? all_rounds * (part + 1) / a.splits : all_rounds) - round0;
 
     ce_pdl_launch_dependents();
     if (threadIdx.x == 0) {
@@ -975,94 +1022,99 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_pair_kernel(const __grid_cons
     uint32_t tmem = tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
-            // ---- producer (in each CTA): its 128 weight rows (and the up rows for SwiGLU), its half of the
-            // tokens, into its own shared memory; the bytes of BOTH CTAs are counted on the leader's barrier
-            ce_pdl_wait();
-            int s = 0, issued = 0;
-            uint32_t ph = 0;                 // parity of the phase of empty_bar[s] that frees the stage's previous use
-            bool ok = true, wrapped = false;
-            for (int tile = pair; tile < total && ok; tile += n_pairs) {
-                int n0 = (tile / tiles_m) * (2 * ROWS_N) + rank * ROWS_N, m0 = (tile % tiles_m) * BN + rank * HALF_N;
-                for (int r = 0; r < rounds; ++r) {
-                    if (wrapped) ok = mbar_wait_cluster(&empty_bar[s], ph ^ 1);
-                    if (!ok) break;
-                    uint32_t bar = map_to_cta(smem_u32(&full_bar[s]), 0);
-                    if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * STAGE_BYTES);
+        // ---- producer (in each CTA): its 128 weight rows (and the up rows for SwiGLU), its half of the
+        // tokens, into its own shared memory; the bytes of BOTH CTAs are counted on the leader's barrier
+        ce_pdl_wait();
+        int s = 0, issued = 0;
+        uint32_t ph = 0;                 // parity of the phase of empty_bar[s] that frees the stage's previous use
+        bool ok = true, wrapped = false;
+        for (int tile = pair; tile < total && ok; tile += n_pairs) {
+            int n0 = (tile / tiles_m) * (2 * ROWS_N) + rank * ROWS_N, m0 = (tile % tiles_m) * btok + rank * half_n;
+            for (int r = 0; r < rounds; ++r) {
+                if (wrapped) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&empty_bar[s], ph ^ 1));
+                if (!ok) break;
+                if (elect_one()) {
+                    uint32_t bar = map_to_cta(smem_u32(&full_bar[s]), leader);
+                    if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * stage_bytes);
 #pragma unroll
                     for (int j = 0; j < KSUB; ++j) {
-                        unsigned char* st = tiles + (size_t)s * STAGE_BYTES + j * SUB_BYTES;
-                        int kx = (r * KSUB + j) * BK;
+                        unsigned char* st = tiles + (size_t)s * stage_bytes + j * sub_bytes;
+                        int kx = ((round0 + r) * KSUB + j) * BK;
                         tma_load_2d_pair(st, &map_w, bar, kx, n0);          // GU: a box of 64 gate rows ...
                         if (GU) tma_load_2d_pair(st + W_BYTES / 2, &map_w, bar, kx, a.N + n0);   // ... and the 64 up rows below them
                         tma_load_2d_pair(st + W_BYTES, &map_x, bar, kx, m0);
                     }
-                    ++issued;
-                    if (++s == stages) { s = 0; ph ^= 1; wrapped = true; }
                 }
-            }
-            if (!ok) {
-                // give the copies in flight time to land before the block may leave (the leader's barriers
-                // count the bytes of both blocks; the peer cannot wait on them, so it waits by the clock)
-                atomicExch(a.status, 51);
-                if (rank == 0) for (int i = max(0, issued - stages); i < issued; ++i) mbar_wait_cluster(&full_bar[i % stages], (i / stages) & 1);
-                else for (int i = 0; i < 64; ++i) __nanosleep(1000);
+                __syncwarp();
+                ++issued;
+                if (++s == stages) { s = 0; ph ^= 1; wrapped = true; }
             }
         }
+        if (!ok && lane == 0) {
+            // give the copies in flight time to land before the block may leave (the leader's barriers
+            // count the bytes of both blocks; the peer cannot wait on them, so it waits by the clock)
+            atomicExch(a.status, 51);
+            if (rank == 0) for (int i = max(0, issued - stages); i < issued; ++i) mbar_wait_cluster(&full_bar[i % stages], (i / stages) & 1);
+            else for (int i = 0; i < 64; ++i) __nanosleep(1000);
+        }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
-            // ---- leader: MMAs for both CTAs.  This one thread's instruction stream is the critical path
+        if (rank == 0) {
+            // ---- leader: MMAs for both CTAs.  This warp's instruction stream is the critical path
             // (a barrier test alone takes about a hundred cycles), so the next stage's barrier is tested
             // BEFORE this stage's MMAs are issued: the test's latency passes while they are queued.
             int lt = 0, s = 0;
             uint32_t ph = 0;
             bool ok = true;
-            uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
+            uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(btok >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
             const uint64_t desc_hi = umma_desc(0);
             bool ready = false;
             for (int tile = pair; tile < total && ok; tile += n_pairs, ++lt) {
                 int buf = lt & 1;
-                if (lt >= 2) ok = mbar_wait_cluster(&acc_empty[buf], ((lt >> 1) - 1) & 1);   // both epilogues have drained this set
-                if (!ok) { atomicExch(a.status, 52); break; }
+                if (lt >= 2) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&acc_empty[buf], ((lt >> 1) - 1) & 1));   // both epilogues have drained this set
+                if (!ok) { if (lane == 0) atomicExch(a.status, 52); break; }
                 uint32_t d_tmem = tmem + buf * ACC_COLS;
                 for (int r = 0; r < rounds; ++r) {
-                    if (!ready) ok = mbar_wait_cluster(&full_bar[s], ph);
-                    if (!ok) { atomicExch(a.status, 53); break; }
+                    if (!ready) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&full_bar[s], ph));
+                    if (!ok) { if (lane == 0) atomicExch(a.status, 53); break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     int sn = s + 1 == stages ? 0 : s + 1;
                     uint32_t phn = sn == 0 ? ph ^ 1 : ph;
-                    ready = mbar_test_cluster(&full_bar[sn], phn);
+                    ready = __all_sync(0xffffffffu, mbar_test_cluster(&full_bar[sn], phn));
+                    if (elect_one()) {
 #pragma unroll
-                    for (int j = 0; j < KSUB; ++j) {
-                        uint32_t st = (base + s * STAGE_BYTES + j * SUB_BYTES) >> 4;
+                        for (int j = 0; j < KSUB; ++j) {
+                            uint32_t st = (base + s * stage_bytes + j * sub_bytes) >> 4;
 #pragma unroll
-                        for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-                            uint64_t bdesc = desc_hi | (uint64_t)((st + ((W_BYTES + kk * UMMA_K * 2) >> 4)) & 0x3FFF);
-                            uint32_t acc = (r > 0 || j > 0 || kk > 0) ? 1u : 0u;
-                            umma2_bf16(d_tmem, desc_hi | (uint64_t)((st + ((kk * UMMA_K * 2) >> 4)) & 0x3FFF), bdesc, idesc, acc);
+                            for (int kk = 0; kk < BK / UMMA_K; ++kk) {
+                                uint64_t bdesc = desc_hi | (uint64_t)((st + ((W_BYTES + kk * UMMA_K * 2) >> 4)) & 0x3FFF);
+                                uint32_t acc = (r > 0 || j > 0 || kk > 0) ? 1u : 0u;
+                                umma2_bf16(d_tmem, desc_hi | (uint64_t)((st + ((kk * UMMA_K * 2) >> 4)) & 0x3FFF), bdesc, idesc, acc);
+                            }
                         }
+                        umma2_commit_both(&empty_bar[s], leader);     // the stage is free in both CTAs
                     }
-                    umma2_commit_both(&empty_bar[s]);     // the stage is free in both CTAs
+                    __syncwarp();
                     s = sn; ph = phn;
                 }
-                if (ok) umma2_commit_both(&acc_full[buf]);
+                if (ok && elect_one()) umma2_commit_both(&acc_full[buf], leader);
+                __syncwarp();
             }
         }
-    } else {
+    } else if (!SPLIT) {
         // ---- epilogue (in each CTA): its own 128 rows
         int quad = warp & 3;
         int row = quad * 32 + lane;
         ce_pdl_wait();
         int lt = 0;
         bool ok = true;
-        uint32_t leader_empty[2] = {map_to_cta(smem_u32(&acc_empty[0]), 0), map_to_cta(smem_u32(&acc_empty[1]), 0)};
+        uint32_t leader_empty[2] = {map_to_cta(smem_u32(&acc_empty[0]), leader), map_to_cta(smem_u32(&acc_empty[1]), leader)};
         for (int tile = pair; tile < total && ok; tile += n_pairs, ++lt) {
             int buf = lt & 1;
             int n = (tile / tiles_m) * (2 * ROWS_N) + rank * ROWS_N + (GU ? (row & 63) : row);
             bool up_row = GU && row >= 64;
             const float bg = CLAMP ? gate_bias(a, n, 0) : 0.f, bu = CLAMP ? gate_bias(a, n, 1) : 0.f;
-            int m0 = (tile % tiles_m) * BN;
-            int m_valid = min(BN, a.M - m0);
+            int m0 = (tile % tiles_m) * btok;
+            int m_valid = min(btok, a.M - m0);
             const bool accum = !GU && a.mode == TC_ACCUM_F32 && n < a.N;
             float xv[32];
             if (accum) {       // the residual values of the first 32 tokens are on their way before the accumulators are ready
@@ -1081,7 +1133,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_pair_kernel(const __grid_cons
             if (!GU && a.mode == TC_ACCUM_F32) {
                 // x += product, 32 tokens a chunk; the next chunk's residual values are loaded while this one is stored
 #pragma unroll 1
-                for (int c = 0; c < BN; c += 32) {
+                for (int c = 0; c < btok; c += 32) {
                     if (c >= m_valid) break;
                     float g[32], xn[32];
                     tmem_ld32(taddr + c, g);
@@ -1098,7 +1150,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_pair_kernel(const __grid_cons
                 }
             } else
 #pragma unroll 1
-            for (int c = 0; c < BN; c += 32) {
+            for (int c = 0; c < btok; c += 32) {
                 if (c >= m_valid) break;
                 float g[32];
                 tmem_ld32(taddr + c, g);
@@ -1129,7 +1181,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_pair_kernel(const __grid_cons
                 if (n < a.N) {
 #pragma unroll
                     for (int j = 0; j < 32; ++j)
-                        if (c + j < m_valid) epilogue_store(a, m0 + c + j, n, g[j], 0.f);
+                        if (c + j < m_valid) store_plain(a, m0 + c + j, n, g[j]);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1137,9 +1189,97 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_pair_kernel(const __grid_cons
             if (threadIdx.x == 64) mbar_arrive_remote(leader_empty[buf]);     // (two arrivals: one per CTA)
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    } else {
+        ce_pdl_wait();
+        if (threadIdx.x == 64) s_acc_ok = rounds == 0 || mbar_wait_cluster(&acc_full[0], 0) ? 1 : 0;
     }
     __syncthreads();
     cluster_sync_all();                              // nobody leaves while the other may still signal it
+    if (SPLIT) {
+        // every MMA of the cluster has completed, so every CTA's stages are free
+        const int quad = warp & 3, row = quad * 32 + lane;
+        const int m0 = (pair % tiles_m) * btok, m_valid = min(btok, a.M - m0);
+        const int per = ((m_valid + a.splits - 1) / a.splits + 15) & ~15;      // tokens a pair finishes: whole chunks of 16
+        const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16);
+        const bool ok = s_acc_ok != 0;
+        if (warp >= 2) {
+            if (!ok && threadIdx.x == 64) atomicExch(a.status, 54);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int q = 0; q < a.splits; ++q) {
+                if (q == part) continue;
+                // [partial][token / 4][row][token % 4]: a warp's 16-byte writes are consecutive
+                const uint32_t dst = map_to_cta(base + (uint32_t)(part < q ? part : part - 1) * (uint32_t)per * 512u + (uint32_t)row * 16u, 2 * q + rank);
+                for (int c = q * per; c < min(m_valid, (q + 1) * per); c += 16) {
+                    float g[16];
+                    tmem_ld16(taddr + c, g);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)((c - q * per) / 4 + i) * 2048u),
+                                     "f"(g[4 * i]), "f"(g[4 * i + 1]), "f"(g[4 * i + 2]), "f"(g[4 * i + 3]) : "memory");
+                }
+            }
+        }
+        __syncwarp();
+        cluster_sync_all();                          // the partial sums are where they are added
+        if (warp >= 2 && ok) {
+            const int n = (pair / tiles_m) * (2 * ROWS_N) + rank * ROWS_N + (GU ? (row & 63) : row);
+            const bool up_row = GU && row >= 64, accum = !GU && a.mode == TC_ACCUM_F32;
+            const float bg = CLAMP ? gate_bias(a, n, 0) : 0.f, bu = CLAMP ? gate_bias(a, n, 1) : 0.f;
+            const int stop = min(m_valid, (part + 1) * per);
+            for (int c = part * per; c < stop; c += 16) {
+                float xv[16];
+                if (accum) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) xv[j] = n < a.N && c + j < stop ? ((const float*)a.out)[(size_t)(m0 + c + j) * a.ldo + n] : 0.f;
+                }
+                float own[16], g[16];
+                tmem_ld16(taddr + c, own);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+#pragma unroll
+                    for (int q = 0; q < PAIR_MAX_SPLITS; ++q) {
+                        if (q >= a.splits) break;
+                        float4 v = make_float4(own[4 * i], own[4 * i + 1], own[4 * i + 2], own[4 * i + 3]);
+                        if (q != part)
+                            v = *reinterpret_cast<const float4*>(tiles + (size_t)(q < part ? q : q - 1) * per * 512 +
+                                                                 (size_t)((c - part * per) / 4 + i) * 2048 + (size_t)row * 16);
+                        g[4 * i] = q ? g[4 * i] + v.x : v.x;
+                        g[4 * i + 1] = q ? g[4 * i + 1] + v.y : v.y;
+                        g[4 * i + 2] = q ? g[4 * i + 2] + v.z : v.z;
+                        g[4 * i + 3] = q ? g[4 * i + 3] + v.w : v.w;
+                    }
+                }
+                if (GU) {
+                    // as above in chunks of 32: the gate thread takes tokens 0..7 of the chunk, the up thread tokens 8..15
+                    float* xg = xbuf + ((c >> 4) & 1) * (2 * 64 * 17) + (row & 63) * 17;
+                    float* xu = xg + 64 * 17;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        if (up_row) xu[j] = g[j];
+                        else xg[j] = g[8 + j];
+                    }
+                    asm volatile("bar.sync 2, 128;" ::: "memory");     // (the buffer used two chunks ago has been read by then)
+                    const int t0 = up_row ? 8 : 0;
+                    __nv_bfloat16* op = (__nv_bfloat16*)a.out + (size_t)(m0 + c + t0) * a.ldo + n;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float gate = up_row ? xg[j] : g[j], upv = up_row ? g[8 + j] : xu[j];
+                        if (n < a.N && c + t0 + j < stop) op[(size_t)j * a.ldo] = __float2bfloat16_rn(gated_mul_fast<CLAMP>(a, gate, upv, bg, bu));
+                    }
+                } else if (n < a.N) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        if (c + j >= stop) continue;
+                        if (accum) ((float*)a.out)[(size_t)(m0 + c + j) * a.ldo + n] = xv[j] + g[j];
+                        else store_plain(a, m0 + c + j, n, g[j]);
+                    }
+                }
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        cluster_sync_all();                          // (a pair's tensor memory is given back when both of its CTAs are done)
+    }
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
@@ -1213,50 +1353,103 @@ int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, const TcArgs
     return ce_check_launch("ce_gemm_tc (persistent)");
 }
 
-template <int BN, bool GU, int KSUB, bool CLAMP = false>
-int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, const TcArgs& a, int tiles_n, int tiles_m, cudaStream_t stream) {
-    constexpr size_t stage = KSUB * (BM * BK * 2 + (BN / 2) * BK * 2);
-    int stages = (int)((200 * 1024) / stage);
-    if (stages > 8) stages = 8;
-    size_t smem = stages * stage + 1024;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<BN, GU, KSUB, CLAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_gemm_tc: %s", cudaGetErrorString(e));
-        attr_set = true;
-    }
-    long long total = (long long)tiles_n * tiles_m;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * (ce_sm_count() / 2));
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    // Tiles are dealt to pairs in a fixed stride, so every pair has to be resident at once: not every
-    // SM can be paired (a cluster lies within one GPC), so ask how many pairs fit.
-    static int max_pairs = 0;
-    if (max_pairs == 0) {
+// Whole stages in what an SM's 227 KB leave beside the static part (the gated epilogue's exchange buffer) and the alignment.
+constexpr size_t pair_budget(bool gu) { return (gu ? 207 : 224) * 1024; }
+int pair_stages(int btok, bool gu) {
+    int stages = (int)(pair_budget(gu) / pair_stage_bytes(btok));
+    return stages > PAIR_MAX_STAGES ? PAIR_MAX_STAGES : stages;
+}
+
+// How many clusters of `splits` pairs are resident at once (not every SM can be paired: a cluster lies within one GPC).
+template <bool GU, int KSUB, bool CLAMP, bool SPLIT>
+int pair_clusters(int splits) {
+    static int resident[PAIR_MAX_SPLITS + 1];
+    if (resident[splits] == 0) {
+        const size_t smem = pair_budget(GU) + 1024;
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<GU, KSUB, CLAMP, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(2 * splits * (ce_sm_count() / (2 * splits)));
+        cfg.blockDim = dim3(THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 2 * splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int n = 0;
-        cudaError_t e = cudaOccupancyMaxActiveClusters(&n, gemm_tc_pair_kernel<BN, GU, KSUB, CLAMP>, &cfg);
-        if (e != cudaSuccess || n < 1) return ce_fail(CE_ERR_CUDA, "ce_gemm_tc (pairs): no resident cluster: %s", cudaGetErrorString(e));
-        max_pairs = n;
-        if (getenv("CE_GEMM_TRACE")) fprintf(stderr, "[carbon_engine_b200] gemm pairs<%d,%d>: %d resident\n", BN, (int)GU, n);
+        e = cudaOccupancyMaxActiveClusters(&n, gemm_tc_pair_kernel<GU, KSUB, CLAMP, SPLIT>, &cfg);
+        if (e != cudaSuccess || n < 1) return 0;
+        resident[splits] = n;
+        if (getenv("CE_GEMM_TRACE")) fprintf(stderr, "[carbon_engine_b200] gemm pairs<%d,%d,%d> x %d: %d resident\n", (int)GU, KSUB, (int)SPLIT, splits, n);
     }
-    int pairs = max_pairs;
-    if (total < pairs) pairs = (int)total;
-    cfg.gridDim = dim3(2 * pairs);
+    return resident[splits];
+}
+
+// The persistent kernel deals its tiles in a fixed stride, so every pair has to be resident at once; with SPLIT there is a cluster a
+// tile, and a cluster needs no other.
+template <bool GU, int KSUB, bool CLAMP, bool SPLIT>
+int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, TcArgs a, int tiles_n, int tiles_m, int btok, cudaStream_t stream) {
+    const int stages = pair_stages(btok, GU), resident = pair_clusters<GU, KSUB, CLAMP, SPLIT>(a.splits);
+    if (resident < 1) return ce_fail(CE_ERR_CUDA, "ce_gemm_tc (pairs): no resident cluster of %d: %s", 2 * a.splits, cudaGetErrorString(cudaGetLastError()));
+    const long long total = (long long)tiles_n * tiles_m;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * a.splits * (unsigned)(SPLIT || total < resident ? total : resident));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = (size_t)stages * pair_stage_bytes(btok) + 1024;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2 * a.splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ce_pdl_enabled() ? 2 : 1;
-    ce_note("gemm_tc_pair_kernel");
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<BN, GU, KSUB, CLAMP>, mw, mx, a, stages, tiles_n, tiles_m);
+    ce_note(SPLIT ? "gemm_tc_pair_kernel (split-K in a cluster)" : "gemm_tc_pair_kernel");
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_pair_kernel<GU, KSUB, CLAMP, SPLIT>, mw, mx, a, stages, tiles_n, tiles_m, btok);
     if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_gemm_tc (pairs): %s", cudaGetErrorString(e));
     return ce_check_launch("ce_gemm_tc (pairs)");
+}
+
+template <bool GU, bool CLAMP>
+int launch_pair_any(const CUtensorMap& mw, const CUtensorMap& mx, const TcArgs& a, int tiles_n, int tiles_m, int btok, cudaStream_t stream) {
+    if (pair_ksub(btok) == 1)
+        return a.splits > 1 ? launch_pair<GU, 1, CLAMP, true>(mw, mx, a, tiles_n, tiles_m, btok, stream)
+                            : launch_pair<GU, 1, CLAMP, false>(mw, mx, a, tiles_n, tiles_m, btok, stream);
+    return a.splits > 1 ? launch_pair<GU, 2, CLAMP, true>(mw, mx, a, tiles_n, tiles_m, btok, stream)
+                        : launch_pair<GU, 2, CLAMP, false>(mw, mx, a, tiles_n, tiles_m, btok, stream);
+}
+
+// Tokens of a tile and pairs that share its K, for a product of `rows` tiles of weight rows: the least time by a model.  128 k of a
+// tile take 0.39 us at 80 tokens, 0.445 at 128 and 0.75 at 256 (measured with all pairs busy); a wave of tiles takes its rounds, or
+// what its weights take from memory; beside that a launch costs 5.5 us, and 5.3 more where the pairs of a cluster add their sums.
+// A second wave of clusters is worse than any plan without (a cluster starts when all of its SMs are free).  A plan has to be 4 %
+// better than a wider tile to replace it: padding costs power too.  Measured (us, 4,096 features of K = 4,096 / 12,288, and 12,288
+// gated; one pair a tile of 128 or 256 tokens -> planned):
+//     130 tokens: 25 / 56 / 58 -> 17 / 30 / 57;   512: 25 / 59 / 85 -> 22 / 47 / 84;   1,733: 58 / 145 / 251 -> 51 / 136 / 246
+struct PairPlan {
+    int btok, splits;
+};
+template <bool GU>
+PairPlan plan_pairs(long long rows, int M, int K) {
+    const double rounds = (K + 2 * BK - 1) / (2 * BK);
+    PairPlan best{PAIR_MAX_TOKENS, 1};
+    double least = 1e30;
+    for (int btok = PAIR_MAX_TOKENS; btok >= 80; btok -= 16) {
+        const long long tiles_m = (M + btok - 1) / btok, tiles = rows * tiles_m;
+        const double tile_us = rounds * (0.445 + (btok > 128 ? 0.00238 : 0.0011) * (btok - 128)), tile_bytes = 4.0 * BM * K / tiles_m;
+        const bool wide = pair_ksub(btok) == 1;
+        for (int s = 1; s <= PAIR_MAX_SPLITS; ++s) {
+            const int at_once = s == 1 ? (wide ? pair_clusters<GU, 1, false, false>(1) : pair_clusters<GU, 2, false, false>(1))
+                                       : (wide ? pair_clusters<GU, 1, false, true>(s) : pair_clusters<GU, 2, false, true>(s));
+            if (at_once < 1 || (s > 1 && (rounds / s < 4 || tiles > at_once))) continue;
+            const long long full = tiles / at_once, rest = tiles % at_once;
+            const double us = full * fmax(tile_us / s, at_once * tile_bytes / 6.0e6) + (rest ? fmax(tile_us / s, rest * tile_bytes / 6.0e6) : 0.) +
+                              (s == 1 ? 5.5 : 10.8);
+            if (us < 0.96 * least) { least = us; best = PairPlan{btok, s}; }
+        }
+    }
+    return best;
 }
 
 }  // namespace
@@ -1358,27 +1551,19 @@ extern "C" int ce_gemm_tc(const void* A, const void* W, void* C, int M, int N, i
         TcArgs pa{C, scratch, counters, status, M, N, K, ldc, mode, 1, kblocks, kblocks, ptrace, 0, 0, bias, limit, alpha};
         static int use_pairs = getenv("CE_GEMM_NO_PAIRS") ? 0 : 1;
         if (use_pairs && N >= 2 * BM) {     // CTA pairs: 256 weight rows a tile, each CTA loads half of the tokens
-            // SwiGLU: 128 gate rows and their 128 up rows a pair tile (boxes of 64 rows), 256 tokens as well
-            // 256 tokens a tile, or 128 where that needs clearly fewer waves of pairs (a few hundred tokens):
-            // waves x time of a tile decides; a tile of 128 tokens takes 0.75 of the time of one of 256 (measured)
+            // SwiGLU: 128 gate rows and their 128 up rows a pair tile (boxes of 64 rows)
             long long rows_t = nacc == 2 ? (N + BM - 1) / BM : (N + 2 * BM - 1) / (2 * BM);
-            long long n_pairs = ce_sm_count() / 2;
-            long long t256 = rows_t * ((M + 255) / 256), t128 = rows_t * ((M + 127) / 128);
-            double c256 = (double)((t256 + n_pairs - 1) / n_pairs), c128 = (double)((t128 + n_pairs - 1) / n_pairs) * 0.75;
-            int ptok = c128 < c256 ? 128 : 256;
+            const PairPlan plan = nacc == 2 ? plan_pairs<true>(rows_t, M, K) : plan_pairs<false>(rows_t, M, K);
             CUtensorMap px2, pw2;
-            if ((prc = get_map(A, M, K, lda, ptok / 2, &px2))) return prc;
-            long long ptiles_m = (M + ptok - 1) / ptok;
+            if ((prc = get_map(A, M, K, lda, plan.btok / 2, &px2))) return prc;
+            const int ptiles_m = (M + plan.btok - 1) / plan.btok;
+            pa.splits = plan.splits;
             if (nacc == 2) {
                 if ((prc = get_map(W, (long long)N * 2, K, K, BM / 2, &pw2))) return prc;
-                if (mode == TC_CLAMPGLU)
-                    return ptok == 128 ? launch_pair<128, true, 2, true>(pw2, px2, pa, (int)rows_t, (int)ptiles_m, stream)
-                                       : launch_pair<256, true, 2, true>(pw2, px2, pa, (int)rows_t, (int)ptiles_m, stream);
-                return ptok == 128 ? launch_pair<128, true, 2>(pw2, px2, pa, (int)rows_t, (int)ptiles_m, stream)
-                                   : launch_pair<256, true, 2>(pw2, px2, pa, (int)rows_t, (int)ptiles_m, stream);
+                return mode == TC_CLAMPGLU ? launch_pair_any<true, true>(pw2, px2, pa, (int)rows_t, ptiles_m, plan.btok, stream)
+                                           : launch_pair_any<true, false>(pw2, px2, pa, (int)rows_t, ptiles_m, plan.btok, stream);
             }
-            return ptok == 128 ? launch_pair<128, false, 2>(pw, px2, pa, (int)rows_t, (int)ptiles_m, stream)
-                               : launch_pair<256, false, 2>(pw, px2, pa, (int)rows_t, (int)ptiles_m, stream);
+            return launch_pair_any<false, false>(pw, px2, pa, (int)rows_t, ptiles_m, plan.btok, stream);
         }
         if (mode == TC_CLAMPGLU) return launch_persistent<128, 2, true>(pw, px, pa, (int)tiles_n, (int)tiles_m, stream);
         return nacc == 2 ? launch_persistent<128, 2>(pw, px, pa, (int)tiles_n, (int)tiles_m, stream)
