@@ -177,16 +177,25 @@ __device__ __forceinline__ void epilogue_store(const TcArgs& a, int m, int n, fl
     else ((__nv_bfloat16*)a.out)[o] = __float2bfloat16_rn(gated_mul<CLAMP>(a, v, up, CLAMP ? gate_bias(a, n, 0) : 0.f, CLAMP ? gate_bias(a, n, 1) : 0.f));
 }
 
-// The same without the gated activations, for epilogues that are unrolled over tokens: a block runs its epilogue once, so every
-// instruction of it is fetched from L2 first, and the activations' code, repeated for every token and never run, cost the store of
-// 130 x 4,096 results 6 us (two pairs a tile: 24 us, where adding into the residual took 18).
-__device__ __forceinline__ void store_plain(const TcArgs& a, int m, int n, float v) {
-    const size_t o = (size_t)m * a.ldo + n;
-    if (a.mode == TC_ACCUM_F32) ((float*)a.out)[o] += v;
-    else if (a.mode == TC_STORE_F32) ((float*)a.out)[o] = v;
-    else {
-        const float r = fmaxf(v, 0.f);
-        ((__nv_bfloat16*)a.out)[o] = __float2bfloat16_rn(a.mode == TC_RELU2 ? r * r : v);
+// Tokens m .. m + n_tok - 1 (at most CNT) of feature n, stored in bfloat16 (squared relu first, mode 5) or float32: the epilogues
+// that neither add into the residual nor are gated.  A block runs its epilogue once, so every instruction of it is fetched from L2
+// first: with the gated activations' code in it, repeated for every token and never run, the store of 130 x 4,096 results took 6 us
+// more (24 us, where adding into the residual took 18); with a test of the mode for every token, that of 512 x 6,144 took 5 us more.
+template <int CNT>
+__device__ __forceinline__ void store_tokens(const TcArgs& a, int m, int n, const float (&g)[CNT], int n_tok) {
+    if (a.mode == TC_STORE_F32) {
+        float* o = (float*)a.out + (size_t)m * a.ldo + n;
+#pragma unroll
+        for (int j = 0; j < CNT; ++j)
+            if (j < n_tok) o[(size_t)j * a.ldo] = g[j];
+    } else {
+        __nv_bfloat16* o = (__nv_bfloat16*)a.out + (size_t)m * a.ldo + n;
+        const bool square = a.mode == TC_RELU2;
+#pragma unroll
+        for (int j = 0; j < CNT; ++j) {
+            const float r = fmaxf(g[j], 0.f);
+            if (j < n_tok) o[(size_t)j * a.ldo] = __float2bfloat16_rn(square ? r * r : g[j]);
+        }
     }
 }
 
@@ -210,7 +219,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_tc_kernel(const __grid_consta
     uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char* tiles = smem_raw + (base - smem_u32(smem_raw));
 
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     int n0 = blockIdx.x * (GU ? BM / 2 : BM), m0 = blockIdx.y * BN, split = blockIdx.z;
     int kb0 = split * a.kblocks_per_split;
     int kb1 = min(kb0 + a.kblocks_per_split, a.kblocks);
@@ -284,24 +293,24 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_tc_kernel(const __grid_consta
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // ---- MMA issuer
-            uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-            bool ok = true, ready = false;
-            int s = 0;
-            uint32_t ph = 0;
-            const uint64_t desc_hi = umma_desc(0);
-            for (int i = 0; i < nkb; ++i) {
-                // this thread's instruction stream bounds a block's rate when few blocks share the weights:
-                // no divisions, and the next stage's barrier is tested before this stage's MMAs are issued
-                if (!ready) ok = mbar_wait(&full_bar[s], ph);
-                if (!ok) break;
-                if (tracing && i == 0) s_rec[2] = gtime();
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                int sn = s + 1 == stages ? 0 : s + 1;
-                uint32_t phn = sn == 0 ? ph ^ 1 : ph;
-                ready = i + 1 < nkb && mbar_try_wait(&full_bar[sn], phn);
-                uint32_t st = (base + s * STAGE_BYTES) >> 4;
+        // ---- MMA issuer: the whole warp walks the loop, one elected lane issues (see elect_one)
+        uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+        bool ok = true, ready = false;
+        int s = 0;
+        uint32_t ph = 0;
+        const uint64_t desc_hi = umma_desc(0);
+        for (int i = 0; i < nkb; ++i) {
+            // this warp's instruction stream bounds a block's rate when few blocks share the weights:
+            // no divisions, and the next stage's barrier is tested before this stage's MMAs are issued
+            if (!ready) ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[s], ph));
+            if (!ok) break;
+            if (tracing && i == 0 && lane == 0) s_rec[2] = gtime();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            int sn = s + 1 == stages ? 0 : s + 1;
+            uint32_t phn = sn == 0 ? ph ^ 1 : ph;
+            ready = __all_sync(0xffffffffu, i + 1 < nkb && mbar_try_wait(&full_bar[sn], phn));
+            uint32_t st = (base + s * STAGE_BYTES) >> 4;
+            if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < BK / UMMA_K; ++kk) {
                     uint64_t bdesc = desc_hi | (uint64_t)((st + ((W_BYTES + kk * UMMA_K * 2) >> 4)) & 0x3FFF);
@@ -309,13 +318,17 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_tc_kernel(const __grid_consta
                     umma_bf16(tmem, desc_hi | (uint64_t)((st + ((kk * UMMA_K * 2) >> 4)) & 0x3FFF), bdesc, idesc, acc);
                 }
                 umma_commit(&empty_bar[s]);          // the stage is free once these MMAs have read it
-                s = sn; ph = phn;
             }
+            __syncwarp();
+            s = sn; ph = phn;
+        }
+        if (elect_one()) {
             if (ok) umma_commit(&acc_bar);           // the accumulators are complete
             else { atomicExch(a.status, 5); atomicExch(&s_abort, 1); }
             if (tracing) s_rec[3] = gtime();
             if (a.trace) atomicMax(&g_trace_all[(a.trace & 255) * 4 + 0], gtime());
         }
+        __syncwarp();
     } else {
         // ---- epilogue: 4 warps, each reads the 32 accumulator lanes of its quadrant
         int quad = warp & 3;
@@ -386,9 +399,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_tc_kernel(const __grid_consta
                             for (int j = 0; j < 16; ++j)
                                 if (c + j < m_valid) xp[(size_t)j * a.ldo] = xv[j] + g[j];
                         } else {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                if (c + j < m_valid) store_plain(a, m0 + c + j, n, g[j]);
+                            store_tokens(a, m0 + c, n, g, m_valid - c);
                         }
                     }
                 }
@@ -506,11 +517,12 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_tc_kernel(const __grid_consta
                                 for (int j = 0; j < TB; ++j) g[j] += tg[s][j];
                             }
                         }
+                        if (a.mode == TC_ACCUM_F32) {
 #pragma unroll
-                        for (int j = 0; j < TB; ++j) {
-                            if (mb + j >= m_hi) continue;
-                            if (a.mode == TC_ACCUM_F32) ((float*)a.out)[(size_t)(m0 + mb + j) * a.ldo + n] = xv[j] + g[j];
-                            else store_plain(a, m0 + mb + j, n, g[j]);
+                            for (int j = 0; j < TB; ++j)
+                                if (mb + j < m_hi) ((float*)a.out)[(size_t)(m0 + mb + j) * a.ldo + n] = xv[j] + g[j];
+                        } else {
+                            store_tokens(a, m0 + mb, n, g, m_hi - mb);
                         }
                     }
                 }
@@ -557,7 +569,7 @@ __global__ void __launch_bounds__(THREADS, 2) gemm_tc_kernel(const __grid_consta
                         float* xp = (float*)a.out + (size_t)(m0 + m) * a.ldo + n;
                         *xp = *xp + g;
                     } else {
-                        store_plain(a, m0 + m, n, g);
+                        epilogue_store(a, m0 + m, n, g, 0.f);
                     }
                 }
             }
@@ -884,12 +896,13 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_persistent_kernel(const __gri
                         for (int j = 0; j < 32; ++j)
                             if (c + j < m_valid) xp[(size_t)j * a.ldo] = xv[j] + g[j];
                     } else {
+                        if (NACC == 2) {
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (c + j < m_valid) {
-                                if (NACC == 2) epilogue_store<CLAMP>(a, m0 + c + j, n, g[j], u[j]);
-                                else store_plain(a, m0 + c + j, n, g[j]);
-                            }
+                            for (int j = 0; j < 32; ++j)
+                                if (c + j < m_valid) epilogue_store<CLAMP>(a, m0 + c + j, n, g[j], u[j]);
+                        } else {
+                            store_tokens(a, m0 + c, n, g, m_valid - c);
+                        }
                     }
                 }
             }
@@ -1178,11 +1191,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_pair_kernel(const __grid_cons
                     }
                     continue;
                 }
-                if (n < a.N) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        if (c + j < m_valid) store_plain(a, m0 + c + j, n, g[j]);
-                }
+                if (n < a.N) store_tokens(a, m0 + c, n, g, m_valid - c);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -1267,11 +1276,12 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_pair_kernel(const __grid_cons
                         if (n < a.N && c + t0 + j < stop) op[(size_t)j * a.ldo] = __float2bfloat16_rn(gated_mul_fast<CLAMP>(a, gate, upv, bg, bu));
                     }
                 } else if (n < a.N) {
+                    if (accum) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        if (c + j >= stop) continue;
-                        if (accum) ((float*)a.out)[(size_t)(m0 + c + j) * a.ldo + n] = xv[j] + g[j];
-                        else store_plain(a, m0 + c + j, n, g[j]);
+                        for (int j = 0; j < 16; ++j)
+                            if (c + j < stop) ((float*)a.out)[(size_t)(m0 + c + j) * a.ldo + n] = xv[j] + g[j];
+                    } else {
+                        store_tokens(a, m0 + c, n, g, stop - c);
                     }
                 }
             }
@@ -1421,8 +1431,9 @@ int launch_pair_any(const CUtensorMap& mw, const CUtensorMap& mx, const TcArgs& 
 }
 
 // Tokens of a tile and pairs that share its K, for a product of `rows` tiles of weight rows: the least time by a model.  128 k of a
-// tile take 0.39 us at 80 tokens, 0.445 at 128 and 0.75 at 256 (measured with all pairs busy); a wave of tiles takes its rounds, or
-// what its weights take from memory; beside that a launch costs 5.5 us, and 5.3 more where the pairs of a cluster add their sums.
+// tile take 0.425 us at 80 tokens, 0.445 at 128 and 0.75 at 256 (measured with all pairs busy); a wave of tiles takes its rounds, or
+// what its weights take from memory; beside that a launch costs 5.5 us, and 5 to 8 more where the
+// pairs of a cluster add their sums.
 // A second wave of clusters is worse than any plan without (a cluster starts when all of its SMs are free).  A plan has to be 4 %
 // better than a wider tile to replace it: padding costs power too.  Measured (us, 4,096 features of K = 4,096 / 12,288, and 12,288
 // gated; one pair a tile of 128 or 256 tokens -> planned):
@@ -1437,7 +1448,7 @@ PairPlan plan_pairs(long long rows, int M, int K) {
     double least = 1e30;
     for (int btok = PAIR_MAX_TOKENS; btok >= 80; btok -= 16) {
         const long long tiles_m = (M + btok - 1) / btok, tiles = rows * tiles_m;
-        const double tile_us = rounds * (0.445 + (btok > 128 ? 0.00238 : 0.0011) * (btok - 128)), tile_bytes = 4.0 * BM * K / tiles_m;
+        const double tile_us = rounds * (0.445 + (btok > 128 ? 0.00238 : 0.0004) * (btok - 128)), tile_bytes = 4.0 * BM * K / tiles_m;
         const bool wide = pair_ksub(btok) == 1;
         for (int s = 1; s <= PAIR_MAX_SPLITS; ++s) {
             const int at_once = s == 1 ? (wide ? pair_clusters<GU, 1, false, false>(1) : pair_clusters<GU, 2, false, false>(1))
@@ -1445,7 +1456,7 @@ PairPlan plan_pairs(long long rows, int M, int K) {
             if (at_once < 1 || (s > 1 && (rounds / s < 4 || tiles > at_once))) continue;
             const long long full = tiles / at_once, rest = tiles % at_once;
             const double us = full * fmax(tile_us / s, at_once * tile_bytes / 6.0e6) + (rest ? fmax(tile_us / s, rest * tile_bytes / 6.0e6) : 0.) +
-                              (s == 1 ? 5.5 : 10.8);
+                              (s == 1 ? 5.5 : 7.8 + 1.5 * s);
             if (us < 0.96 * least) { least = us; best = PairPlan{btok, s}; }
         }
     }
