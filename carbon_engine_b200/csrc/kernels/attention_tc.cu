@@ -367,16 +367,19 @@ __global__ void __launch_bounds__(THREADS) attention_prefill_tc_kernel(const __g
             float m_new = raise ? m_tile : m_run;
             float m_use = m_new == -INFINITY ? 0.f : m_new;
             float alpha = raise ? ce_exp2_fast(m_run - m_use) : 1.0f;
-            float sum = 0.f, sum1 = 0.f;
+            // pairs of scores: fma.f32x2 and add.f32x2 are two IEEE operations an instruction (the same results)
+            float2 sum2 = make_float2(0.f, 0.f);
             uint32_t packed[BN / 2];
+            const float2 scale2 = make_float2(a.scale_log2, a.scale_log2), minus_m = make_float2(-m_use, -m_use);
 #pragma unroll
             for (int i = 0; i < BN; i += 2) {
-                float p0 = ce_exp2_fast(BIAS ? sv[i] - m_use : fmaf(sv[i], a.scale_log2, -m_use));
-                float p1 = ce_exp2_fast(BIAS ? sv[i + 1] - m_use : fmaf(sv[i + 1], a.scale_log2, -m_use));
-                sum += p0; sum1 += p1;
-                packed[i / 2] = pack2(p0, p1);
+                const float2 x = make_float2(sv[i], sv[i + 1]);
+                const float2 t = BIAS ? __fadd2_rn(x, minus_m) : __ffma2_rn(x, scale2, minus_m);
+                const float2 p = make_float2(ce_exp2_fast(t.x), ce_exp2_fast(t.y));
+                sum2 = __fadd2_rn(sum2, p);
+                packed[i / 2] = pack2(p.x, p.y);
             }
-            sum += sum1;
+            const float sum = sum2.x + sum2.y;
             l_run = l_run * alpha + sum;
             m_run = m_new;
             // P and (if a scale was raised) O may be touched only after the previous PV product is complete

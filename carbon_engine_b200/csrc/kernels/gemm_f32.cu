@@ -202,8 +202,13 @@ template <int TM, int LM, int TN, bool GATED, bool VEC>
 int f32_launch(const F32Args& a, dim3 grid, int stages, cudaStream_t stream) {
     constexpr int BM = TM * LM;
     const size_t smem = sizeof(float) * ((size_t)stages * (BM + F_ROWS) * FK + (size_t)BM * F_PITCH);
-    cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<TM, LM, TN, GATED, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_gemm_plain: %s", cudaGetErrorString(e));
+    cudaError_t e;
+    static bool attr_set = false;                          // (the number of stages, so the size, is the tile's)
+    if (!attr_set) {
+        e = cudaFuncSetAttribute(gemm_f32_kernel<TM, LM, TN, GATED, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_gemm_plain: %s", cudaGetErrorString(e));
+        attr_set = true;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(F_THREADS);
