@@ -11,7 +11,9 @@
 // output tile, optionally over a slice of K (split-K, used
 // when there are fewer tiles than SMs).  For SwiGLU the 128 rows of a tile are 64 gate rows and the 64 up
 // rows of the same features (two TMA boxes), so it is one product with one accumulator like the others,
-// and it is never split.  More tokens: persistent kernels further down (CTA pairs with cta_group::2).
+// and this kernel never splits it.  More tokens: CTA pairs with cta_group::2 further down (where tiles are
+// few and the tokens at most 512, the pairs of a cluster share a tile's K, gated or not), and a persistent
+// kernel of single CTAs for outputs of less than 256 columns.
 // Warp 0 issues the TMA loads, warp 1 owns tensor memory and issues the MMAs, warps 2-5 read the
 // accumulators back (tcgen05.ld) and run the epilogue.  With split-K every CTA writes its partial
 // sums to scratch memory; the CTA that arrives last for a tile adds the partials in split order
@@ -1435,32 +1437,48 @@ int launch_pair_any(const CUtensorMap& mw, const CUtensorMap& mx, const TcArgs& 
 // what its weights take from memory; beside that a launch costs 5.5 us, and 5 to 8 more where the
 // pairs of a cluster add their sums.
 // A second wave of clusters is worse than any plan without (a cluster starts when all of its SMs are free).  A plan has to be 4 %
-// better than a wider tile to replace it: padding costs power too.  Measured (us, 4,096 features of K = 4,096 / 12,288, and 12,288
-// gated; one pair a tile of 128 or 256 tokens -> planned):
-//     130 tokens: 25 / 56 / 58 -> 17 / 30 / 57;   512: 25 / 59 / 85 -> 22 / 47 / 84;   1,733: 58 / 145 / 251 -> 51 / 136 / 246
+// better than a wider tile to replace it: padding costs power too.  Measured (us, weights from memory; 4,096 features of K = 4,096 /
+// 12,288, and 12,288 gated; one pair a tile of 128 or 256 tokens, issued by single threads -> as it is):
+//     130 tokens: 25 / 54 / 62 -> 21 / 36 / 59;   512: 26 / 57 / 87 -> 24 / 51 / 86;   1,733: 54 / 138 / 250 -> 49 / 126 / 244
 struct PairPlan {
     int btok, splits;
 };
-template <bool GU>
-PairPlan plan_pairs(long long rows, int M, int K) {
+// at_once[s]: clusters of s pairs that run side by side
+PairPlan model_pairs(long long rows, int M, int K, int splits_lo, int splits_hi, const int* at_once) {
     const double rounds = (K + 2 * BK - 1) / (2 * BK);
-    PairPlan best{PAIR_MAX_TOKENS, 1};
+    PairPlan best{PAIR_MAX_TOKENS, splits_lo};
     double least = 1e30;
     for (int btok = PAIR_MAX_TOKENS; btok >= 80; btok -= 16) {
         const long long tiles_m = (M + btok - 1) / btok, tiles = rows * tiles_m;
         const double tile_us = rounds * (0.445 + (btok > 128 ? 0.00238 : 0.0004) * (btok - 128)), tile_bytes = 4.0 * BM * K / tiles_m;
-        const bool wide = pair_ksub(btok) == 1;
-        for (int s = 1; s <= PAIR_MAX_SPLITS; ++s) {
-            const int at_once = s == 1 ? (wide ? pair_clusters<GU, 1, false, false>(1) : pair_clusters<GU, 2, false, false>(1))
-                                       : (wide ? pair_clusters<GU, 1, false, true>(s) : pair_clusters<GU, 2, false, true>(s));
-            if (at_once < 1 || (s > 1 && (rounds / s < 4 || tiles > at_once))) continue;
-            const long long full = tiles / at_once, rest = tiles % at_once;
-            const double us = full * fmax(tile_us / s, at_once * tile_bytes / 6.0e6) + (rest ? fmax(tile_us / s, rest * tile_bytes / 6.0e6) : 0.) +
+        for (int s = splits_lo; s <= splits_hi; ++s) {
+            const int n = at_once[s];
+            if (s > 1 && (rounds / s < 4 || tiles > n)) continue;
+            const long long full = tiles / n, rest = tiles % n;
+            const double us = full * fmax(tile_us / s, n * tile_bytes / 6.0e6) + (rest ? fmax(tile_us / s, rest * tile_bytes / 6.0e6) : 0.) +
                               (s == 1 ? 5.5 : 7.8 + 1.5 * s);
             if (us < 0.96 * least) { least = us; best = PairPlan{btok, s}; }
         }
     }
     return best;
+}
+
+// How many pairs share K is a function of N, K and the band of the tokens (up to 256, up to 512; more never share): it is taken from
+// the plan for the band's largest step on a chip with the clusters below side by side, whatever this chip's answer is.  So a token's
+// sums are taken in the same order in every step of a band and on every chip.  (B200s differ in their GPCs: the one measured holds
+// 74, 33, 22 and 15 clusters; on one that holds fewer the last of them wait, and the sums stay.)  The tile's tokens, which no sum
+// depends on, follow the step.  Sharing only up to 256 tokens, which leaves one band less, was slower (4,096 features of K = 12,288,
+// 300 / 400 / 512 tokens: 39 / 43 / 50 -> 49 / 49 / 51 us).
+template <bool GU>
+PairPlan plan_pairs(long long rows, int M, int K) {
+    static const int assumed[PAIR_MAX_SPLITS + 1] = {0, 74, 32, 20, 14};
+    const int band = M <= PAIR_MAX_TOKENS ? PAIR_MAX_TOKENS : 2 * PAIR_MAX_TOKENS;
+    int splits = M <= band ? model_pairs(rows, band, K, 1, PAIR_MAX_SPLITS, assumed).splits : 1;
+    if (splits > 1 && (pair_clusters<GU, 1, false, true>(splits) < 1 || pair_clusters<GU, 2, false, true>(splits) < 1))
+        splits = 1;                                         // (a part of a chip that has no room for even one such cluster)
+    int at_once[PAIR_MAX_SPLITS + 1] = {};
+    at_once[splits] = splits > 1 ? assumed[splits] : pair_clusters<GU, 2, false, false>(1);
+    return at_once[splits] > 0 ? model_pairs(rows, M, K, splits, splits, at_once) : PairPlan{PAIR_MAX_TOKENS, 1};
 }
 
 }  // namespace
@@ -1488,8 +1506,9 @@ static bool pairs_from_129(int M, int N, int nacc) {
     return M <= 256 && M >= pair_min_tokens && N >= 2 * BM && pair_tiles >= pair_min_tiles && !no_pairs;
 }
 
-// How many splits of K a product of these sizes uses (it depends on N and K only while the tokens
-// fit one tile, so a token's sums are taken in the same order whatever else is in the batch).
+// How many splits of K gemm_tc_kernel uses for a product of these sizes, 1 where the pairs take it (it depends on N and K only
+// while the tokens fit one tile, so a token's sums are taken in the same order whatever else is in the batch; the pairs' own
+// sharing of K needs no scratch memory, see plan_pairs).
 extern "C" int ce_gemm_tc_tile_tokens(int M);
 extern "C" int ce_gemm_tc_splits(int M, int N, int K) {
     int kblocks = (K + BK - 1) / BK;
@@ -1550,7 +1569,7 @@ extern "C" int ce_gemm_tc(const void* A, const void* W, void* C, int M, int N, i
     int nacc = TC_GATED(mode) ? 2 : 1;
     int kblocks = (K + BK - 1) / BK;
     bool early_pairs = pairs_from_129(M, N, nacc);
-    if (M > 256 || early_pairs) {       // many tokens: the persistent kernels, no split-K
+    if (M > 256 || early_pairs) {       // many tokens: the pairs (K shared in a cluster up to 512 tokens: plan_pairs), or one CTA a tile
         int pbn = nacc == 2 ? 128 : 256;
         long long tiles_m = (M + pbn - 1) / pbn, tiles_n = (N + BM - 1) / BM;
         if (tiles_m * tiles_n > 2147483647LL) return ce_fail(CE_ERR_SIZE, "ce_gemm_tc: too many tiles");

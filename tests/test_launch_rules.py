@@ -1,0 +1,88 @@
+"""The rules by which the launchers choose grids, clusters and attributes, on the CPU: the kernels' objects linked with a runtime that
+records launches (fake_cudart.cpp)."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from carbon_engine_b200.csrc import build
+
+STORE, ACCUM, SWIGLU, CLAMPGLU = 0, 2, 3, 6
+ADDR = 1 << 20                     # an aligned address that nothing reads
+
+
+class Launch(ctypes.Structure):
+    _fields_ = [("grid", ctypes.c_uint * 3), ("block", ctypes.c_uint * 3), ("cluster", ctypes.c_uint * 3), ("smem", ctypes.c_uint),
+                ("dependent", ctypes.c_uint), ("device", ctypes.c_int), ("kernel", ctypes.c_char * 256)]
+
+
+@pytest.fixture(scope="module")
+def linked(tmp_path_factory):
+    try:
+        nvcc = build._nvcc()
+    except build.BuildError:
+        pytest.skip("no CUDA toolkit")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+    headers = build._sources(build.KERNEL_DIR, (".cuh", ".h"))
+    names = ("errors", "tensor_map", "gemm_tc", "gemm_f32", "gemm_plain", "attention_f32")
+    objects = build._compile_all(nvcc, build.NVCC_FLAGS, [os.path.join(build.KERNEL_DIR, n + ".cu") for n in names], headers, build.build_dir(), "k")
+    out = str(tmp_path_factory.mktemp("fake") / "libfake.so")
+    cxx = os.environ.get("CXX") or shutil.which("g++") or shutil.which("c++")
+    source = os.path.join(os.path.dirname(os.path.abspath(__file__)), "fake_cudart.cpp")
+    subprocess.run([cxx, "-shared", "-fPIC", "-std=c++17", "-I", cuda, source] + objects + ["-o", out], check=True)
+    return out
+
+
+class Chip:
+    """A process's first look at a chip: every instance loads a copy of the library, with nothing kept from other instances."""
+
+    count = 0
+
+    def __init__(self, linked, room):
+        Chip.count += 1
+        copy = f"{linked}.{Chip.count}.so"
+        shutil.copy(linked, copy)
+        self.lib = ctypes.CDLL(copy, mode=os.RTLD_LOCAL | os.RTLD_NOW | getattr(os, "RTLD_DEEPBIND", 0))
+        self.lib.ce_last_error.restype = ctypes.c_char_p
+        for blocks, clusters in room.items():
+            self.lib.fake_room(blocks, clusters)
+
+    def _launched(self, code):
+        assert code == 0, self.lib.ce_last_error().decode()
+        seen = Launch()
+        self.lib.fake_last(ctypes.byref(seen))
+        return seen
+
+    def gemm_tc(self, M, N, K, mode=STORE):
+        p = ctypes.c_void_p(ADDR)
+        return self._launched(self.lib.ce_gemm_tc(p, p, p, M, N, K, K, N, mode, p, ctypes.c_longlong(1 << 40), p, 1 << 20, p, None,
+                                                  ctypes.c_float(0), ctypes.c_float(0), None))
+
+
+B200 = {2: 74, 4: 33, 6: 22, 8: 15}
+OTHER = {2: 74, 4: 30, 6: 17, 8: 12}
+# weight rows and K of this engine's products at several widths, gated ones among them
+PRODUCTS = [(4096, 4096, STORE), (4096, 12288, ACCUM), (6144, 4096, STORE), (3072, 9728, ACCUM), (5120, 17408, ACCUM), (3840, 8192, STORE),
+            (8448, 8192, STORE), (3328, 16384, ACCUM), (2048, 4096, SWIGLU), (1536, 8192, CLAMPGLU), (12288, 4096, SWIGLU)]
+
+
+def parts(launch):
+    assert b"gemm_tc_pair_kernel" in launch.kernel
+    return launch.cluster[0] // 2
+
+
+@pytest.mark.parametrize("N,K,mode", PRODUCTS)
+def test_the_pairs_that_share_k_depend_on_the_weights_alone(linked, N, K, mode):
+    """A token's sums are taken in the same order in every step of a band of tokens, on every chip, and in one piece beyond 512 tokens."""
+    here, there = Chip(linked, B200), Chip(linked, OTHER)
+    for band in ((129, 130, 160, 176, 203, 224, 255, 256), (257, 300, 336, 400, 448, 511, 512)):
+        assert len({parts(chip.gemm_tc(M, N, K, mode)) for M in band for chip in (here, there)}) == 1
+    assert all(parts(chip.gemm_tc(M, N, K, mode)) == 1 for M in (513, 600, 700, 1021, 4096) for chip in (here, there))
+
+
+def test_products_with_few_tiles_share_k(linked):
+    chip = Chip(linked, B200)
+    assert [parts(chip.gemm_tc(200, N, K, mode)) for N, K, mode in PRODUCTS[:6]] == [2, 2, 1, 4, 3, 2]
+    assert [parts(chip.gemm_tc(400, N, K, mode)) for N, K, mode in PRODUCTS[:6]] == [1, 2, 1, 2, 1, 2]
