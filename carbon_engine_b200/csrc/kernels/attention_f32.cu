@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include <type_traits>
 #include <limits.h>
+#include <math.h>
 
 namespace {
 
@@ -71,6 +72,13 @@ __device__ __forceinline__ AfMerge af_merge(float& M, float m) {
     AfMerge f{M == -INFINITY ? 0.f : expf(M - top), m == -INFINITY ? 0.f : expf(m - top)};
     M = top;
     return f;
+}
+// The inverse of a row's sum of exponentials.  A sum of nothing is 0 where the row's own key lies on a page the request does not hold
+// (reported in status); where it was seen, every score was -inf, and the softmax of those is not a number.
+__device__ __forceinline__ float af_inverse(const AttnF32Args& a, const int* table, int position, float sum) {
+    if (sum > 0.f) return 1.0f / sum;
+    const int page = table[position / a.page_size];
+    return page >= 0 && page < a.num_pages ? NAN : 0.f;
 }
 __device__ __forceinline__ float af_join(float total, float part, const AfMerge& f) { return __fmaf_rn(part, f.stripe, __fmul_rn(total, f.before)); }
 
@@ -326,7 +334,7 @@ __global__ void __launch_bounds__(AF_THREADS, 2) attention_f32_kernel(AttnF32Arg
         for (int i = 0; i < RT; ++i) {
             const int r = lm + 8 * i;
             if (r >= rows) continue;
-            const float inv = L[i] > 0.f ? 1.0f / L[i] : 0.f;
+            const float inv = af_inverse(a, table, s_hi[r], L[i]);
             float* out = a.out + ((size_t)(t0 + r / a.group) * a.nh + kvh * a.group + r % a.group) * d;
 #pragma unroll
             for (int j = 0; j < CT; ++j) {
@@ -367,7 +375,7 @@ __global__ void __launch_bounds__(AF_THREADS, 2) attention_f32_kernel(AttnF32Arg
             sum = af_join(sum, l[s], f);
             acc = af_join(acc, x[s], f);
         }
-        const float inv = sum > 0.f ? 1.0f / sum : 0.f;
+        const float inv = af_inverse(a, table, s_hi[r], sum);
         a.out[((size_t)(t0 + r / a.group) * a.nh + kvh * a.group + r % a.group) * d + col] = __fmul_rn(acc, inv);
     }
     af_cluster_sync();                                // no block's stripe goes away while another may still read it

@@ -125,3 +125,21 @@ def test_float32_attention_flags_a_page_the_request_does_not_hold():
     table[0, 5] = -1
     out, st = attention([(199, 1)], torch.randn(1, 16, device=dev()), kp, vp, table, 1, 1, 16, 16, 0, 16)
     assert st == 4 and torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("seqs", [[(30, 1), (0, 1)], [(0, 40), (7, 30)]])
+def test_float32_attention_of_scores_that_are_all_minus_infinity_is_not_a_number(seqs):
+    """Products of finite numbers can overflow.  One row whose scores all do, among rows whose scores do not, alone and in a tile."""
+    from carbon_engine_b200 import ops
+    torch.manual_seed(4)
+    table, kp, vp = paged_layout([c + n for c, n in seqs], 16, 1, 16, torch.float32)
+    for b, (c, n) in enumerate(seqs):
+        fill_pools(kp, vp, table.cpu().numpy(), b, torch.full((c + n, 1, 16), 1e20, device=dev()), torch.randn(c + n, 1, 16, device=dev()), 16)
+    q = torch.randn(sum(n for _, n in seqs), 2 * 16, device=dev()) * 1e-20
+    q[0, 16:] = -1e20
+    got, st = attention(seqs, q, kp, vp, table, 2, 1, 16, 16, 0, 32)
+    positions, seq_of_token, slots = step_meta(seqs)
+    want = torch.empty_like(got)
+    ops.attention_generic(q, 32, kp, vp, want, positions, seq_of_token, slots, table, status(), 2, 1, 16, 16, 0, 0.25)
+    assert st == 0 and torch.equal(got.isnan(), want.isnan())
+    assert got[0, 16:].isnan().all() and not got[1:].isnan().any() and not got[0, :16].isnan().any()
