@@ -39,6 +39,7 @@ struct F32Args {
     float* C;
     int M, N, K, lda, ldc, mode;
     int run, splits;                    // k of a run; blocks a tile's runs are dealt to (1, or one a run)
+    int weights_ready;                  // no kernel in front writes W
     GpGate gate;
 };
 
@@ -98,8 +99,9 @@ __global__ void __launch_bounds__(F_THREADS, 2) gemm_f32_kernel(F32Args a, int s
     auto load_w = [&](int s) { f_load<F_ROWS, VEC>(ring + (s % stages) * STAGE + BM * FK, a.W, a.K, k_begin + s * FK, k_end, w_row); };
     auto load_a = [&](int s) { f_load<BM, VEC>(ring + (s % stages) * STAGE, a.A, a.lda, k_begin + s * FK, k_end, a_row); };
 
-    // no kernel writes weights, so the first stages of them come before the wait for the kernels in front
+    // weights that no kernel writes come before the wait for the kernels in front; any other W is read after it, like A
     ce_pdl_launch_dependents();
+    if (!a.weights_ready) ce_pdl_wait();
     for (int s = 0; s < stages - 1; ++s)
         if (s < slabs) load_w(s);
     ce_pdl_wait();
@@ -243,7 +245,7 @@ int f32_pick(const F32Args& a, dim3 grid, int stages, bool vec, cudaStream_t str
 }  // namespace
 
 int ce_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldc, int mode, const GpGate& gate,
-                cudaStream_t stream) {
+                bool weights_ready, cudaStream_t stream) {
     const int runs = K / 256 < 1 ? 1 : K / 256 > F_MAX_RUNS ? F_MAX_RUNS : K / 256;
     const int run = ((K + runs - 1) / runs + FK - 1) / FK * FK;
     const bool vec = K % 4 == 0 && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
@@ -254,7 +256,7 @@ int ce_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, i
     // 80 tiles, 87 us against 330 on one block a tile); with more it gains nothing (301 tokens, 480 tiles: 448 and 446 us) and
     // later loses (1,000 tokens, 1,536 tiles: 1,193 us on one block a tile, 1,396 in clusters).
     const int splits = runs > 1 && tiles < 2 * ce_sm_count() ? runs : 1;
-    F32Args a{A, W, C, M, N, K, lda, ldc, mode, run, splits, gate};
+    F32Args a{A, W, C, M, N, K, lda, ldc, mode, run, splits, weights_ready, gate};
     dim3 grid((N + features - 1) / features, (M + tokens - 1) / tokens, splits);
     switch (tokens) {
         case 4: return f32_pick<4, 1, 1>(a, grid, 4, vec, stream);

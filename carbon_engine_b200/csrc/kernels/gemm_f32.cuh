@@ -10,6 +10,7 @@ struct GpGate {
     float limit, alpha;
 };
 
-// The product in float32 (sizes and pointers checked by the caller).
+// The product in float32 (sizes and pointers checked by the caller).  weights_ready: no kernel on the stream may still be writing W,
+// so its first rows are read while the kernels in front run.
 int ce_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldc, int mode, const GpGate& gate,
-                cudaStream_t stream);
+                bool weights_ready, cudaStream_t stream);

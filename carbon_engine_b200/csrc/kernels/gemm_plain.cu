@@ -112,16 +112,17 @@ static int launch_plain(const void* A, const void* W, void* C, int M, int N, int
     return ce_check_launch("ce_gemm_plain");
 }
 
-// N is the number of output columns (for SwiGLU: the intermediate width, W having 2N rows).
+// N is the number of output columns (for SwiGLU: the intermediate width, W having 2N rows).  weights_ready: see gemm_f32.cuh (the
+// bfloat16 product always waits for the kernels in front).
 extern "C" int ce_gemm_plain(const void* A, const void* W, void* C, int dtype, int M, int N, int K, int lda, int ldc,
-                             int mode, const float* bias, float limit, float alpha, cudaStream_t stream) {
+                             int mode, const float* bias, float limit, float alpha, int weights_ready, cudaStream_t stream) {
     GpGate gate{bias, limit, alpha};
     if (M == 0 || N == 0) return CE_OK;
     if (!A || !W || !C) return ce_fail(CE_ERR_ARG, "ce_gemm_plain: null pointer");
     if (K <= 0) return ce_fail(CE_ERR_SIZE, "ce_gemm_plain: K=%d", K);
     if ((M + GP_BM - 1) / GP_BM > 65535) return ce_fail(CE_ERR_SIZE, "ce_gemm_plain: M=%d is too large", M);
     if (mode < GP_STORE || mode > GP_CLAMPGLU) return ce_fail(CE_ERR_ARG, "ce_gemm_plain: unknown epilogue %d", mode);
-    if (dtype == CE_F32) return ce_gemm_f32((const float*)A, (const float*)W, (float*)C, M, N, K, lda, ldc, mode, gate, stream);
+    if (dtype == CE_F32) return ce_gemm_f32((const float*)A, (const float*)W, (float*)C, M, N, K, lda, ldc, mode, gate, weights_ready != 0, stream);
     if (dtype == CE_BF16) return launch_plain<__nv_bfloat16>(A, W, C, M, N, K, lda, ldc, mode, gate, stream);
     return ce_fail(CE_ERR_ARG, "ce_gemm_plain: unknown dtype %d", dtype);
 }

@@ -714,8 +714,10 @@ def attention_f32(q, q_stride: int, k_pool, v_pool, out, positions, seq_slot, q_
     return True
 
 
-def gemm_plain(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, mode: int, glu: Optional[GluParams] = None) -> None:
-    """c = a @ w.T with float32 FMA arithmetic; see csrc/kernels/gemm_f32.cuh for the epilogues."""
+def gemm_plain(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, mode: int, glu: Optional[GluParams] = None,
+               weights_ready: bool = False) -> None:
+    """c = a @ w.T with float32 FMA arithmetic; see csrc/kernels/gemm_f32.cuh for the epilogues.  ``weights_ready``: no kernel still
+    running on the stream writes ``w``, so the float32 product may begin to read it while the kernels in front of it run."""
     _need(w, "w", a.dtype); _need(c, "c")
     if a.stride(-1) != 1 or c.stride(-1) != 1:
         raise KernelError("gemm_plain: rows must be contiguous")
@@ -729,7 +731,7 @@ def gemm_plain(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, mode: int, glu
         raise KernelError(f"gemm_plain: output must be {want}")
     bias, limit, alpha = glu_args(glu, mode, N)
     _ok(kernels().ce_gemm_plain(_ptr(a), _ptr(w), _ptr(c), dtype_code(a.dtype), M, N, K, a.stride(0), c.stride(0),
-                                mode, bias, limit, alpha, _stream()))
+                                mode, bias, limit, alpha, int(weights_ready), _stream()))
 
 
 def streams_norm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, eps: float, groups: int = 1,

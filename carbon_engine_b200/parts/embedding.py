@@ -83,7 +83,7 @@ class LMHead(Part):
             return logits
         z = ctx.buffer((R, self.width))
         self.norm.forward(x, z, rows)
-        matmul_nt(z, self.weight, logits, STORE_F32)
+        matmul_nt(z, self.weight, logits, STORE_F32, weights_ready=True)
         if self.logit_cap > 0.0:
             ops.tanh_cap(logits, self.logit_cap)
         return logits

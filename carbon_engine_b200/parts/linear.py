@@ -30,9 +30,10 @@ BF16_BACKEND = "auto"
 PLAIN_MAX_MACS = 1 << 24
 
 
-def matmul_nt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, scratch=None, glu=None) -> None:
+def matmul_nt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, scratch=None, glu=None, weights_ready: bool = False) -> None:
     """out (op)= a @ w.T with the epilogue ``mode``; a [M, K], w [N or 2N, K].  ``glu``: the clamped gated epilogue's limit,
-    factor and bias (``ops.GluParams``)."""
+    factor and bias (``ops.GluParams``).  ``weights_ready``: ``w`` is a loaded weight, which no kernel of a step writes
+    (``ops.gemm_plain``)."""
     if a.shape[0] == 0:
         return
     prof = ops.profiling()
@@ -41,7 +42,7 @@ def matmul_nt(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, sc
         R = w.shape[0]          # weight rows: N, or 2N for SwiGLU
         prof.note_work((M * K + R * K) * a.element_size() + M * out.shape[1] * out.element_size(), 2 * M * R * K)
     if a.dtype == torch.float32 or BF16_BACKEND == "plain":
-        ops.gemm_plain(a, w, out, mode, glu)
+        ops.gemm_plain(a, w, out, mode, glu, weights_ready)
         return
     if BF16_BACKEND in ("auto", "tensor"):
         from .. import ops_tensor
@@ -134,7 +135,7 @@ class Linear(Part):
     def forward(self, a: torch.Tensor, out: torch.Tensor, mode: int = STORE, add_bias: bool = True, glu=None) -> None:
         """``add_bias=False``: the caller adds ``self.bias`` itself (in a kernel that touches the output anyway).  ``glu``: with
         the clamped gated epilogue, its limit, factor and bias."""
-        matmul_nt(a, self.weight, out, mode, glu=glu)
+        matmul_nt(a, self.weight, out, mode, glu=glu, weights_ready=True)
         if mode == CLAMPGLU:
             return
         if add_bias and self.bias is not None and a.shape[0] > 0:

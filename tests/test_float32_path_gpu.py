@@ -61,6 +61,26 @@ def test_float32_product_has_the_same_bits_in_every_tile_and_cluster(N, K):
         assert torch.equal(product(a[lo:lo + n], w, ops.GEMM_STORE), whole[lo:lo + n]), n
 
 
+@pytest.mark.parametrize("M", [3, 40, 100])
+def test_float32_product_reads_a_matrix_that_the_kernel_in_front_makes(M):
+    """The second product's W is the first one's result, with dependent launches on: the first takes some 100 us, the second must not
+    begin to read before it ends."""
+    from carbon_engine_b200 import ops
+    torch.manual_seed(5)
+    a, b, x = torch.randn(1024, 4096, device=dev()), torch.randn(512, 4096, device=dev()), torch.randn(M, 512, device=dev())
+    made = torch.zeros(1024, 512, device=dev())
+    ops.set_dependent_launches(True)
+    ops.gemm_plain(a, b, made, ops.GEMM_STORE)
+    torch.cuda.synchronize()
+    want, got = product(x, made, ops.GEMM_STORE), torch.empty(M, 1024, device=dev())
+    for _ in range(5):
+        made.zero_()
+        torch.cuda.synchronize()
+        ops.gemm_plain(a, b, made, ops.GEMM_STORE)
+        ops.gemm_plain(x, made, got, ops.GEMM_STORE)               # (nothing between the two launches)
+        assert torch.equal(got, want)
+
+
 def attention(seqs, q, kp, vp, table, nh, nkv, d, ps, window, stride):
     from carbon_engine_b200 import ops
     T = sum(n for _, n in seqs)
