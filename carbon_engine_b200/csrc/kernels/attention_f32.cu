@@ -386,13 +386,10 @@ int af_launch(AttnF32Args a, int blocks, bool apart, cudaStream_t stream) {
     if (blocks == 0) return CE_OK;
     const size_t smem = sizeof(float) * ((size_t)(8 * RT + AF_KEYS) * (a.d + 4) + (size_t)AF_KEYS * a.d + (size_t)8 * RT * AF_SP);
     cudaError_t e;
-    static bool attr_set = false;
-    if (!attr_set) {                                       // once, for the largest head size of the instantiation
-        constexpr size_t most = sizeof(float) * ((size_t)(8 * RT + AF_KEYS) * (64 * CT + 4) + (size_t)AF_KEYS * 64 * CT + (size_t)8 * RT * AF_SP);
-        e = cudaFuncSetAttribute(attention_f32_kernel<RT, CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-        if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_attention_f32: %s", cudaGetErrorString(e));
-        attr_set = true;
-    }
+    static std::atomic<unsigned long long> allowed{0};
+    constexpr size_t most = sizeof(float) * ((size_t)(8 * RT + AF_KEYS) * (64 * CT + 4) + (size_t)AF_KEYS * 64 * CT + (size_t)8 * RT * AF_SP);
+    e = ce_allow_smem(allowed, attention_f32_kernel<RT, CT>, most);        // (for the largest head size of the instantiation)
+    if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_attention_f32: %s", cudaGetErrorString(e));
     a.stripes_apart = apart && (long long)blocks * a.nkv < 2 * ce_sm_count();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks, a.nkv, a.stripes_apart ? AF_STRIPES : 1);

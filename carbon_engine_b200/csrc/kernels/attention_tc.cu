@@ -467,12 +467,9 @@ int get_map(const void* ptr, long long rows, long long cols, long long ld, int b
 template <int D, bool BIAS>
 int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const TcAttnArgs& a, dim3 grid, cudaStream_t stream) {
     size_t smem = (size_t)BM * D * 2 + STAGES * 2 * BN * D * 2 + BM * BN * 2 + 192;    // tiles + barriers
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<D, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_attention_prefill_tc: %s", cudaGetErrorString(e));
-        attr_set = true;
-    }
+    static std::atomic<unsigned long long> allowed{0};
+    cudaError_t e = ce_allow_smem(allowed, attention_prefill_tc_kernel<D, BIAS>, smem);
+    if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_attention_prefill_tc: %s", cudaGetErrorString(e));
     { ce_note("attention_prefill_tc_kernel"); ce_launch(attention_prefill_tc_kernel<D, BIAS>, grid, THREADS, smem, stream, mq, mk, mv, a); }
     return ce_check_launch("ce_attention_prefill_tc");
 }

@@ -17,6 +17,7 @@
 #define CE_F32 0
 #define CE_BF16 1
 
+#include <atomic>
 #include <utility>
 
 extern "C" const char* ce_last_error();
@@ -50,6 +51,19 @@ int ce_fail(int code, const char* fmt, ...);
 void ce_note(const char* kernel_name);
 int ce_check_launch(const char* what);
 int ce_sm_count();
+int ce_device();                 // the current device
+
+// The opt-in to more than 48 KB of shared memory belongs to a device: once for each that launches the kernel.  ``done``: a static of
+// the launcher, one for each kernel and size, with a bit for each device (devices from 64 on opt in at every launch).
+template <typename F>
+inline cudaError_t ce_allow_smem(std::atomic<unsigned long long>& done, F kernel, size_t bytes) {
+    const int device = ce_device();
+    const unsigned long long bit = device >= 0 && device < 64 ? 1ull << device : 0;
+    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
+}
 
 // 2^x in one MUFU instruction (relative error about 2^-22; -inf gives 0).  exp2f() costs several
 // instructions around the same MUFU; the bfloat16 attention kernels, whose probabilities are rounded to

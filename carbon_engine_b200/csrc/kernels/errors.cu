@@ -86,6 +86,11 @@ bool ce_pdl_enabled() {
 }
 extern "C" void ce_set_pdl(int on) { g_pdl = on ? 1 : 0; }
 
+int ce_device() {
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess ? dev : 0;
+}
+
 // Multiprocessors of the current device (asked once).
 int ce_sm_count() {
     static int n = 0;

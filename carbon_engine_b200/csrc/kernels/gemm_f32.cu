@@ -205,12 +205,9 @@ int f32_launch(const F32Args& a, dim3 grid, int stages, cudaStream_t stream) {
     constexpr int BM = TM * LM;
     const size_t smem = sizeof(float) * ((size_t)stages * (BM + F_ROWS) * FK + (size_t)BM * F_PITCH);
     cudaError_t e;
-    static bool attr_set = false;                          // (the number of stages, so the size, is the tile's)
-    if (!attr_set) {
-        e = cudaFuncSetAttribute(gemm_f32_kernel<TM, LM, TN, GATED, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_gemm_plain: %s", cudaGetErrorString(e));
-        attr_set = true;
-    }
+    static std::atomic<unsigned long long> allowed{0};     // (the number of stages, so the size, is the tile's)
+    e = ce_allow_smem(allowed, gemm_f32_kernel<TM, LM, TN, GATED, VEC>, smem);
+    if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_gemm_plain: %s", cudaGetErrorString(e));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(F_THREADS);

@@ -1318,12 +1318,9 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const TcArgs& a, dim3 g
     if (stages > 8) stages = 8;
     if (stages < 2) stages = 2;
     size_t smem = stages * stage + 1024;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, NACC, COOP, CLAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_gemm_tc: %s", cudaGetErrorString(e));
-        attr_set = true;
-    }
+    static std::atomic<unsigned long long> allowed{0};
+    cudaError_t e = ce_allow_smem(allowed, gemm_tc_kernel<BN, NACC, COOP, CLAMP>, smem);
+    if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_gemm_tc: %s", cudaGetErrorString(e));
     if (a.cluster) {
         if ((size_t)BN * BM * 4 > (size_t)stages * stage)
             return ce_fail(CE_ERR_SIZE, "ce_gemm_tc: the partial tile does not fit the stages");
@@ -1340,7 +1337,7 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const TcArgs& a, dim3 g
         cfg.attrs = attr;
         cfg.numAttrs = ce_pdl_enabled() ? 2 : 1;
         ce_note("gemm_tc_kernel (split-K in a cluster)");
-        cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, NACC, COOP, CLAMP>, mw, mx, a, stages);
+        e = cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, NACC, COOP, CLAMP>, mw, mx, a, stages);
         if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_gemm_tc (cluster of %d): %s", (int)grid.z, cudaGetErrorString(e));
         return ce_check_launch("ce_gemm_tc");
     }
@@ -1354,12 +1351,9 @@ int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, const TcArgs
     int stages = (int)((200 * 1024) / stage);
     if (stages > 8) stages = 8;
     size_t smem = stages * stage + 1024;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<BN, NACC, CLAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 2048);
-        if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_gemm_tc: %s", cudaGetErrorString(e));
-        attr_set = true;
-    }
+    static std::atomic<unsigned long long> allowed{0};
+    cudaError_t e = ce_allow_smem(allowed, gemm_tc_persistent_kernel<BN, NACC, CLAMP>, 227 * 1024 - 2048);
+    if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_gemm_tc: %s", cudaGetErrorString(e));
     long long total = (long long)tiles_n * tiles_m;
     int grid = (int)(total < ce_sm_count() ? total : ce_sm_count());
     { ce_note("gemm_tc_persistent_kernel"); ce_launch(gemm_tc_persistent_kernel<BN, NACC, CLAMP>, grid, THREADS, smem, stream, mw, mx, a, stages, tiles_n, tiles_m); }
@@ -1376,11 +1370,12 @@ int pair_stages(int btok, bool gu) {
 // How many clusters of `splits` pairs are resident at once (not every SM can be paired: a cluster lies within one GPC).
 template <bool GU, int KSUB, bool CLAMP, bool SPLIT>
 int pair_clusters(int splits) {
+    static std::atomic<unsigned long long> allowed{0};
+    const size_t smem = pair_budget(GU) + 1024;
+    cudaError_t e = ce_allow_smem(allowed, gemm_tc_pair_kernel<GU, KSUB, CLAMP, SPLIT>, smem);
+    if (e != cudaSuccess) return 0;
     static int resident[PAIR_MAX_SPLITS + 1];
     if (resident[splits] == 0) {
-        const size_t smem = pair_budget(GU) + 1024;
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<GU, KSUB, CLAMP, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return 0;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(2 * splits * (ce_sm_count() / (2 * splits)));
         cfg.blockDim = dim3(THREADS);
@@ -1653,12 +1648,9 @@ int launch_grouped(const CUtensorMap& mw, const CUtensorMap& mx, const TcGroupAr
     int stages = (int)((100 * 1024) / stage);          // two blocks an SM
     if (stages > 8) stages = 8;
     size_t smem = stages * stage + 1024;
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_grouped_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_gemm_tc_grouped: %s", cudaGetErrorString(e));
-        attr_set = true;
-    }
+    static std::atomic<unsigned long long> allowed{0};
+    cudaError_t e = ce_allow_smem(allowed, gemm_tc_grouped_kernel<BN>, smem);
+    if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_gemm_tc_grouped: %s", cudaGetErrorString(e));
     ce_note("gemm_tc_grouped_kernel");
     ce_launch(gemm_tc_grouped_kernel<BN>, grid, THREADS, smem, stream, mw, mx, a, stages);
     return ce_check_launch("ce_gemm_tc_grouped");

@@ -60,6 +60,15 @@ class Chip:
         return self._launched(self.lib.ce_gemm_tc(p, p, p, M, N, K, K, N, mode, p, ctypes.c_longlong(1 << 40), p, 1 << 20, p, None,
                                                   ctypes.c_float(0), ctypes.c_float(0), None))
 
+    def gemm_f32(self, M, N, K, mode=STORE, weights_ready=1):
+        p = ctypes.c_void_p(ADDR)
+        return self._launched(self.lib.ce_gemm_plain(p, p, p, 0, M, N, K, K, N, mode, None, ctypes.c_float(0), ctypes.c_float(0), weights_ready, None))
+
+    def attention_f32(self, n_decode, n_tiles, heads=16, kv_heads=4, d=128, longest=4096):
+        p = ctypes.c_void_p(ADDR)
+        return self._launched(self.lib.ce_attention_f32(*[p] * 10, n_decode, n_tiles, heads, kv_heads, d, heads * d, 64, 100, 100, 0, longest,
+                                                        ctypes.c_float(1), None))
+
 
 B200 = {2: 74, 4: 33, 6: 22, 8: 15}
 OTHER = {2: 74, 4: 30, 6: 17, 8: 12}
@@ -86,3 +95,14 @@ def test_products_with_few_tiles_share_k(linked):
     chip = Chip(linked, B200)
     assert [parts(chip.gemm_tc(200, N, K, mode)) for N, K, mode in PRODUCTS[:6]] == [2, 2, 1, 4, 3, 2]
     assert [parts(chip.gemm_tc(400, N, K, mode)) for N, K, mode in PRODUCTS[:6]] == [1, 2, 1, 2, 1, 2]
+
+
+@pytest.mark.parametrize("launch", [lambda c: c.gemm_f32(100, 4096, 4096), lambda c: c.attention_f32(0, 40), lambda c: c.gemm_tc(4, 4096, 4096),
+                                    lambda c: c.gemm_tc(200, 4096, 4096), lambda c: c.gemm_tc(2048, 4096, 4096), lambda c: c.gemm_tc(2048, 128, 4096)],
+                         ids=["float32 product", "float32 attention", "one-block product", "shared pairs", "pairs", "single CTAs"])
+def test_kernels_of_much_shared_memory_run_on_every_device_of_a_process(linked, launch):
+    chip = Chip(linked, B200)
+    for device in (0, 1, 0, 70, 71):
+        chip.lib.fake_device(device)
+        seen = launch(chip)
+        assert seen.device == device and seen.smem > 48 * 1024
