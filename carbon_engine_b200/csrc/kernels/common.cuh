@@ -65,6 +65,25 @@ inline cudaError_t ce_allow_smem(std::atomic<unsigned long long>& done, F kernel
     return e;
 }
 
+// How many clusters of a launch's shape an otherwise empty device holds at once; 0: none, or the question failed (which leaves no error
+// behind for the next launch's check).  ``room``: a static of the launcher, one for each kernel and cluster size, with each device's
+// answer, 0 before it is asked and -1 for none.
+struct CeRoom {
+    std::atomic<int> seen[64];
+};
+template <typename F>
+inline int ce_clusters_at_once(CeRoom& room, F kernel, const cudaLaunchConfig_t& cfg) {
+    const int device = ce_device();
+    std::atomic<int>* seen = device >= 0 && device < 64 ? &room.seen[device] : nullptr;
+    int n = seen ? seen->load(std::memory_order_relaxed) : 0;
+    if (n == 0) {
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
+        if (n < 1) n = -1;
+        if (seen) seen->store(n, std::memory_order_relaxed);
+    }
+    return n > 0 ? n : 0;
+}
+
 // 2^x in one MUFU instruction (relative error about 2^-22; -inf gives 0).  exp2f() costs several
 // instructions around the same MUFU; the bfloat16 attention kernels, whose probabilities are rounded to
 // 8 bits of mantissa anyway, are bound by exactly those instructions.

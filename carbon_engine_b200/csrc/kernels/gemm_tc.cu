@@ -1371,27 +1371,22 @@ int pair_stages(int btok, bool gu) {
 template <bool GU, int KSUB, bool CLAMP, bool SPLIT>
 int pair_clusters(int splits) {
     static std::atomic<unsigned long long> allowed{0};
+    static CeRoom room[PAIR_MAX_SPLITS + 1];
     const size_t smem = pair_budget(GU) + 1024;
-    cudaError_t e = ce_allow_smem(allowed, gemm_tc_pair_kernel<GU, KSUB, CLAMP, SPLIT>, smem);
-    if (e != cudaSuccess) return 0;
-    static int resident[PAIR_MAX_SPLITS + 1];
-    if (resident[splits] == 0) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * splits * (ce_sm_count() / (2 * splits)));
-        cfg.blockDim = dim3(THREADS);
-        cfg.dynamicSmemBytes = smem;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2 * splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        e = cudaOccupancyMaxActiveClusters(&n, gemm_tc_pair_kernel<GU, KSUB, CLAMP, SPLIT>, &cfg);
-        if (e != cudaSuccess || n < 1) return 0;
-        resident[splits] = n;
-        if (getenv("CE_GEMM_TRACE")) fprintf(stderr, "[carbon_engine_b200] gemm pairs<%d,%d,%d> x %d: %d resident\n", (int)GU, KSUB, (int)SPLIT, splits, n);
+    if (ce_allow_smem(allowed, gemm_tc_pair_kernel<GU, KSUB, CLAMP, SPLIT>, smem) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
     }
-    return resident[splits];
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * splits * (ce_sm_count() / (2 * splits)));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2 * splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return ce_clusters_at_once(room[splits], gemm_tc_pair_kernel<GU, KSUB, CLAMP, SPLIT>, cfg);
 }
 
 // The persistent kernel deals its tiles in a fixed stride, so every pair has to be resident at once; with SPLIT there is a cluster a
@@ -1399,7 +1394,7 @@ int pair_clusters(int splits) {
 template <bool GU, int KSUB, bool CLAMP, bool SPLIT>
 int launch_pair(const CUtensorMap& mw, const CUtensorMap& mx, TcArgs a, int tiles_n, int tiles_m, int btok, cudaStream_t stream) {
     const int stages = pair_stages(btok, GU), resident = pair_clusters<GU, KSUB, CLAMP, SPLIT>(a.splits);
-    if (resident < 1) return ce_fail(CE_ERR_CUDA, "ce_gemm_tc (pairs): no resident cluster of %d: %s", 2 * a.splits, cudaGetErrorString(cudaGetLastError()));
+    if (resident < 1) return ce_fail(CE_ERR_CUDA, "ce_gemm_tc (pairs): no room for a cluster of %d blocks", 2 * a.splits);
     const long long total = (long long)tiles_n * tiles_m;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * a.splits * (unsigned)(SPLIT || total < resident ? total : resident));

@@ -106,3 +106,12 @@ def test_kernels_of_much_shared_memory_run_on_every_device_of_a_process(linked, 
         chip.lib.fake_device(device)
         seen = launch(chip)
         assert seen.device == device and seen.smem > 48 * 1024
+
+
+@pytest.mark.parametrize("answer", [0, -1])                          # no room, and a question that fails
+def test_a_chip_without_room_for_shared_k_is_asked_once_and_runs(linked, answer):
+    chip = Chip(linked, {2: 4, 4: answer, 6: answer, 8: answer})
+    assert parts(chip.gemm_tc(200, 4096, 4096)) == 1
+    asked = chip.lib.fake_occupancy_calls()
+    assert all(parts(chip.gemm_tc(M, N, 4096)) == 1 for M, N in ((200, 4096), (150, 4096), (250, 3840), (300, 4096)))
+    assert chip.lib.fake_occupancy_calls() == asked
