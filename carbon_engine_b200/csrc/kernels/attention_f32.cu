@@ -45,6 +45,7 @@ struct AttnF32Args {
     int nh, nkv, d, q_stride, page_size, max_pages, num_pages, window;
     int group, tokens;           // query heads of a KV head; tokens of a block's rows
     int stripes_apart;           // 1: the blocks of a cluster take a stripe each
+    int overlap;                 // kernels behind may start before this one ends
     float scale;
 };
 
@@ -85,7 +86,8 @@ __device__ __forceinline__ float af_join(float total, float part, const AfMerge&
 // Rows lane % 8 + 8 i (i < RT) a thread; CT x 4 output columns a thread (d <= 64 CT).
 template <int RT, int CT>
 __global__ void __launch_bounds__(AF_THREADS, 2) attention_f32_kernel(AttnF32Args a) {
-    ce_pdl_begin();
+    if (a.overlap) ce_pdl_launch_dependents();
+    ce_pdl_wait();
     constexpr int ROWS = 8 * RT;
     extern __shared__ __align__(16) float af_mem[];
     const int d = a.d, pitch = d + 4, d4 = d >> 2;
@@ -397,19 +399,28 @@ int af_launch(AttnF32Args a, int blocks, bool apart, cudaStream_t stream) {
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
-    int n = 0;
-    if (a.stripes_apart) {
-        attr[n].id = cudaLaunchAttributeClusterDimension;
-        attr[n].val.clusterDim.x = 1; attr[n].val.clusterDim.y = 1; attr[n].val.clusterDim.z = AF_STRIPES;
-        ++n;
-    }
-    if (ce_pdl_enabled()) {
-        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[n].val.programmaticStreamSerializationAllowed = 1;
-        ++n;
-    }
     cfg.attrs = attr;
-    cfg.numAttrs = n;
+    a.overlap = 1;
+    if (a.stripes_apart) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = AF_STRIPES;
+        cfg.numAttrs = 1;
+        cfg.dynamicSmemBytes = most;                             // (one answer for all head sizes)
+        static CeRoom room;
+        const int at_once = ce_clusters_at_once(room, attention_f32_kernel<RT, CT>, cfg);
+        cfg.dynamicSmemBytes = smem;
+        a.overlap = (long long)blocks * a.nkv <= at_once;        // see ce_clusters_at_once
+        if (at_once == 0) {                                      // (no room for a cluster: the same sums in one block)
+            a.stripes_apart = 0;
+            a.overlap = 1;
+            cfg.gridDim.z = 1;
+            cfg.numAttrs = 0;
+        }
+    }
+    if (a.overlap && ce_pdl_enabled()) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
     ce_note(a.stripes_apart ? "attention_f32_kernel (stripes in a cluster)" : "attention_f32_kernel");
     e = cudaLaunchKernelEx(&cfg, attention_f32_kernel<RT, CT>, a);
     if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_attention_f32: %s", cudaGetErrorString(e));
@@ -441,7 +452,7 @@ extern "C" int ce_attention_f32(const float* q, const float* k_pool, const float
     if (!ce_attention_f32_supported(nh, nkv, d, q_stride) || (((uintptr_t)q | (uintptr_t)k_pool | (uintptr_t)v_pool | (uintptr_t)out) & 15))
         return ce_fail(CE_ERR_SIZE, "ce_attention_f32: %d and %d heads of %d, row stride %d", nh, nkv, d, q_stride);
     AttnF32Args a{q, k_pool, v_pool, out, positions, seq_slot, q_start, block_table, nullptr, status, nh, nkv, d, q_stride, page_size,
-                  max_pages, num_pages, window, nh / nkv, 1, 0, scale};
+                  max_pages, num_pages, window, nh / nkv, 1, 0, 1, scale};
     int rc = af_pick(a, a.group, n_decode, true, stream);
     if (rc) return rc;
     a.tiles = tiles;

@@ -67,7 +67,8 @@ inline cudaError_t ce_allow_smem(std::atomic<unsigned long long>& done, F kernel
 
 // How many clusters of a launch's shape an otherwise empty device holds at once; 0: none, or the question failed (which leaves no error
 // behind for the next launch's check).  ``room``: a static of the launcher, one for each kernel and cluster size, with each device's
-// answer, 0 before it is asked and -1 for none.
+// answer, 0 before it is asked and -1 for none.  A launch of more clusters than that stands alone: neither it nor the kernel behind it
+// starts early, since a grid of clusters whose dependents waited beside it was seen not to end (large steps of the CTA pairs).
 struct CeRoom {
     std::atomic<int> seen[64];
 };

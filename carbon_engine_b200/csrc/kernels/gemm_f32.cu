@@ -40,6 +40,7 @@ struct F32Args {
     int M, N, K, lda, ldc, mode;
     int run, splits;                    // k of a run; blocks a tile's runs are dealt to (1, or one a run)
     int weights_ready;                  // no kernel in front writes W
+    int overlap;                        // kernels behind may start before this one ends
     GpGate gate;
 };
 
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(F_THREADS, 2) gemm_f32_kernel(F32Args a, int s
     auto load_a = [&](int s) { f_load<BM, VEC>(ring + (s % stages) * STAGE, a.A, a.lda, k_begin + s * FK, k_end, a_row); };
 
     // weights that no kernel writes come before the wait for the kernels in front; any other W is read after it, like A
-    ce_pdl_launch_dependents();
+    if (a.overlap) ce_pdl_launch_dependents();
     if (!a.weights_ready) ce_pdl_wait();
     for (int s = 0; s < stages - 1; ++s)
         if (s < slabs) load_w(s);
@@ -201,7 +202,7 @@ __global__ void __launch_bounds__(F_THREADS, 2) gemm_f32_kernel(F32Args a, int s
 }
 
 template <int TM, int LM, int TN, bool GATED, bool VEC>
-int f32_launch(const F32Args& a, dim3 grid, int stages, cudaStream_t stream) {
+int f32_launch(F32Args a, dim3 grid, int stages, cudaStream_t stream) {
     constexpr int BM = TM * LM;
     const size_t smem = sizeof(float) * ((size_t)stages * (BM + F_ROWS) * FK + (size_t)BM * F_PITCH);
     cudaError_t e;
@@ -214,19 +215,24 @@ int f32_launch(const F32Args& a, dim3 grid, int stages, cudaStream_t stream) {
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
-    int n = 0;
-    if (a.splits > 1) {
-        attr[n].id = cudaLaunchAttributeClusterDimension;
-        attr[n].val.clusterDim.x = 1; attr[n].val.clusterDim.y = 1; attr[n].val.clusterDim.z = a.splits;
-        ++n;
-    }
-    if (ce_pdl_enabled()) {
-        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[n].val.programmaticStreamSerializationAllowed = 1;
-        ++n;
-    }
     cfg.attrs = attr;
-    cfg.numAttrs = n;
+    a.overlap = 1;
+    if (a.splits > 1) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = a.splits;
+        cfg.numAttrs = 1;
+        static CeRoom room[F_MAX_RUNS + 1];
+        const int at_once = ce_clusters_at_once(room[a.splits], gemm_f32_kernel<TM, LM, TN, GATED, VEC>, cfg);
+        a.overlap = (long long)grid.x * grid.y <= at_once;       // see ce_clusters_at_once
+        if (at_once == 0) {                                      // (no room for a cluster: the same sums on one block a tile)
+            a.splits = cfg.gridDim.z = a.overlap = 1;
+            cfg.numAttrs = 0;
+        }
+    }
+    if (a.overlap && ce_pdl_enabled()) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
     ce_note(a.splits > 1 ? "gemm_f32_kernel (runs of K in a cluster)" : "gemm_f32_kernel");
     e = cudaLaunchKernelEx(&cfg, gemm_f32_kernel<TM, LM, TN, GATED, VEC>, a, stages);
     if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_gemm_plain: %s", cudaGetErrorString(e));
@@ -253,7 +259,7 @@ int ce_gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, i
     // 80 tiles, 87 us against 330 on one block a tile); with more it gains nothing (301 tokens, 480 tiles: 448 and 446 us) and
     // later loses (1,000 tokens, 1,536 tiles: 1,193 us on one block a tile, 1,396 in clusters).
     const int splits = runs > 1 && tiles < 2 * ce_sm_count() ? runs : 1;
-    F32Args a{A, W, C, M, N, K, lda, ldc, mode, run, splits, weights_ready, gate};
+    F32Args a{A, W, C, M, N, K, lda, ldc, mode, run, splits, weights_ready, 1, gate};
     dim3 grid((N + features - 1) / features, (M + tokens - 1) / tokens, splits);
     switch (tokens) {
         case 4: return f32_pick<4, 1, 1>(a, grid, 4, vec, stream);

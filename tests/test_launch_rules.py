@@ -70,7 +70,7 @@ class Chip:
                                                         ctypes.c_float(1), None))
 
 
-B200 = {2: 74, 4: 33, 6: 22, 8: 15}
+B200 = {2: 74, 3: 60, 4: 33, 5: 30, 6: 22, 7: 20, 8: 15}
 OTHER = {2: 74, 4: 30, 6: 17, 8: 12}
 # weight rows and K of this engine's products at several widths, gated ones among them
 PRODUCTS = [(4096, 4096, STORE), (4096, 12288, ACCUM), (6144, 4096, STORE), (3072, 9728, ACCUM), (5120, 17408, ACCUM), (3840, 8192, STORE),
@@ -115,3 +115,23 @@ def test_a_chip_without_room_for_shared_k_is_asked_once_and_runs(linked, answer)
     asked = chip.lib.fake_occupancy_calls()
     assert all(parts(chip.gemm_tc(M, N, 4096)) == 1 for M, N in ((200, 4096), (150, 4096), (250, 3840), (300, 4096)))
     assert chip.lib.fake_occupancy_calls() == asked
+
+
+@pytest.mark.parametrize("room,overlaps", [(2000, True), (16, True), (15, False), (1, False)])
+def test_more_clusters_than_the_chip_holds_stand_alone(linked, room, overlaps):
+    """The float32 kernels: 16 tiles of 128 rows, 4 tokens x 4 KV heads."""
+    chip = Chip(linked, {8: room})
+    for seen in (chip.gemm_f32(4, 2048, 2048), chip.attention_f32(4, 0)):
+        assert seen.cluster[2] == seen.grid[2] == 8 and bool(seen.dependent) == overlaps
+
+
+def test_without_room_for_a_cluster_the_float32_kernels_run_without(linked):
+    chip = Chip(linked, {8: 0})
+    for seen in (chip.gemm_f32(4, 2048, 2048), chip.attention_f32(4, 0)):
+        assert seen.cluster[2] == seen.grid[2] == 1 and seen.dependent
+
+
+@pytest.mark.parametrize("launch", [lambda c: c.gemm_f32(100, 65536, 2048), lambda c: c.attention_f32(0, 64)])
+def test_grids_without_clusters_overlap(linked, launch):
+    seen = launch(Chip(linked, {8: 1}))
+    assert seen.cluster[2] == 1 and seen.dependent
