@@ -441,7 +441,7 @@ extern "C" int ce_attention_f32_supported(int nh, int nkv, int d, int q_stride) 
 }
 
 // The first n_decode sequences of the step bring one token each; tiles: (sequence, first token) pairs that cover the others 64
-// tokens at a time; max_ctx: the longest sequence, these tokens included.
+// tokens at a time; max_ctx: the longest of those others, its new tokens included.
 extern "C" int ce_attention_f32(const float* q, const float* k_pool, const float* v_pool, float* out, const int* positions,
                                 const int* seq_slot, const int* q_start, const int* block_table, const int* tiles, int* status,
                                 int n_decode, int n_tiles, int nh, int nkv, int d, int q_stride, int page_size, int max_pages,

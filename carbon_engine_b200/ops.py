@@ -702,7 +702,7 @@ def attention_generic(q, q_stride: int, k_pool, v_pool, out, positions, seq_of_t
 def attention_f32(q, q_stride: int, k_pool, v_pool, out, positions, seq_slot, q_start, block_table, tiles, status, n_decode: int,
                   n_tiles: int, nh: int, nkv: int, d: int, page_size: int, window: int, max_ctx: int, scale: float) -> bool:
     """Float32 attention of a step: its first ``n_decode`` sequences bring one token each, ``tiles`` ((sequence, first token) pairs)
-    cover the others 64 tokens at a time; ``max_ctx``: the longest sequence's keys.  False if the sizes or layouts are not the kernel's (:func:`attention_generic` takes them)."""
+    cover the others 64 tokens at a time; ``max_ctx``: the keys of the longest of those others.  False if the sizes or layouts are not the kernel's (:func:`attention_generic` takes them)."""
     if any(t.dtype != torch.float32 for t in (q, k_pool, v_pool, out)) or not kernels().ce_attention_f32_supported(nh, nkv, d, q_stride) or \
             (q.data_ptr() | k_pool.data_ptr() | v_pool.data_ptr() | out.data_ptr()) & 15:
         return False

@@ -37,9 +37,10 @@ class AttentionPlan:
     that bring more than one token, 64 and 128 tokens at a time, as (sequence, first token) pairs on
     the device, and the grid bound of the split-KV decode kernel."""
 
-    def __init__(self, tiles, n_tiles, tiles128, n_tiles128, decode_splits):
+    def __init__(self, tiles, n_tiles, tiles128, n_tiles128, decode_splits, portion_ctx=0):
         self.tiles, self.n_tiles, self.tiles128, self.n_tiles128 = tiles, n_tiles, tiles128, n_tiles128
         self.decode_splits = decode_splits       # >= ceil(longest one-token sequence's context / positions per split)
+        self.portion_ctx = portion_ctx           # keys of the longest sequence that brings more than one token
         self.graph_key = decode_splits
 
 
@@ -101,12 +102,13 @@ class PagedAttention(Mixer):
         h_tiles = ctx.bufs.host_section("paged_attention.tiles")
         h_tiles_tc = ctx.bufs.host_section("paged_attention.tiles_tc")
         nt = nt_tc = 0
-        longest = 1
+        longest, portion_ctx = 1, 0
         for b in range(ctx.B):
             n = ctx.h_q_start[b + 1] - ctx.h_q_start[b]
             if b < ctx.n_decode:
                 longest = max(longest, ctx.h_ctx_before[b] + 1)
                 continue
+            portion_ctx = max(portion_ctx, ctx.h_ctx_before[b] + n)
             for q0 in range(0, n, self.TILE):
                 h_tiles[2 * nt], h_tiles[2 * nt + 1] = b, q0
                 nt += 1
@@ -116,7 +118,7 @@ class PagedAttention(Mixer):
         per_split = ops_tensor.decode_split()
         return AttentionPlan(ctx.bufs.dev_section("paged_attention.tiles"), nt,
                              ctx.bufs.dev_section("paged_attention.tiles_tc"), nt_tc,
-                             split_bucket((longest + per_split - 1) // per_split))
+                             split_bucket((longest + per_split - 1) // per_split), portion_ctx)
 
     def forward(self, ctx, h: torch.Tensor, x: torch.Tensor, cache, accumulate: bool = True) -> None:
         T = h.shape[0]
@@ -156,7 +158,7 @@ class PagedAttention(Mixer):
         plan = ctx.plans[self.plan_key]
         if qkv.dtype == torch.float32 and ops.attention_f32(
                 qkv, qkv.shape[1], cache.k_pool, cache.v_pool, out, ctx.positions, ctx.seq_slot, ctx.q_start, table, plan.tiles,
-                ctx.status, ctx.n_decode, plan.n_tiles, nh, nkv, d, cache.page_size, self.window, ctx.max_ctx, self.scale):
+                ctx.status, ctx.n_decode, plan.n_tiles, nh, nkv, d, cache.page_size, self.window, plan.portion_ctx, self.scale):
             return
         ops.attention_generic(qkv, qkv.shape[1], cache.k_pool, cache.v_pool, out, ctx.positions, ctx.seq_of_token,
                               ctx.seq_slot, table, ctx.status, nh, nkv, d, cache.page_size, self.window, self.scale)

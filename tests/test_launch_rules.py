@@ -4,6 +4,7 @@ import ctypes
 import os
 import shutil
 import subprocess
+from types import SimpleNamespace
 
 import pytest
 
@@ -135,3 +136,24 @@ def test_without_room_for_a_cluster_the_float32_kernels_run_without(linked):
 def test_grids_without_clusters_overlap(linked, launch):
     seen = launch(Chip(linked, {8: 1}))
     assert seen.cluster[2] == 1 and seen.dependent
+
+
+@pytest.mark.parametrize("past,clustered", [(0, False), (900, True)])
+def test_a_long_decoding_request_leaves_a_short_prompt_its_plan(linked, monkeypatch, past, clustered):
+    """150 tokens of a prompt after `past`, beside a request that decodes at 5,000."""
+    import torch
+    from carbon_engine_b200 import ops, ops_tensor
+    from carbon_engine_b200.parts.attention import PagedAttention
+    monkeypatch.setattr(ops_tensor, "decode_split", lambda: 128)
+    sections, asked = {}, []
+    bufs = SimpleNamespace(host_section=lambda name: sections.setdefault(name, [0] * 64), dev_section=lambda name: sections[name])
+    ctx = SimpleNamespace(bufs=bufs, B=2, n_decode=1, h_q_start=[0, 1, 151], h_ctx_before=[5000, past], max_ctx=5001, plans={},
+                          positions=None, seq_slot=None, q_start=None, status=None)
+    mixer = PagedAttention(2048, 16, 4, 128, "m")
+    ctx.plans[mixer.plan_key] = mixer.plan_step(ctx)
+    monkeypatch.setattr(ops, "attention_f32", lambda *args: asked.append(args) or True)
+    mixer.attend(ctx, torch.empty(151, 3072), None, SimpleNamespace(k_pool=None, v_pool=None, page_size=64), None)
+    (*_, n_decode, n_tiles, nh, nkv, d, page_size, window, longest, scale), = asked
+    assert (n_decode, n_tiles, window) == (1, 3, 0)
+    seen = Chip(linked, {8: 1000}).attention_f32(0, n_tiles, longest=longest)
+    assert (seen.cluster[2] == 8) == clustered
