@@ -73,7 +73,7 @@ def run() -> int:
         ang = torch.arange(64, dtype=torch.float64)[:, None] * inv[None]
         cos, sin = ang.cos().float().to(dev), ang.sin().float().to(dev)
         qw, kw = 1 + 0.1 * torch.randn(d, device=dev), 1 + 0.1 * torch.randn(d, device=dev)
-        outs = []
+        outs, outs_f32 = [], []
         for lo, hi in ((0, 30), (30, 44), (44, 45)):
             n = hi - lo
             mk = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
@@ -84,6 +84,12 @@ def run() -> int:
             ops.attention_generic(qkv, qkv.shape[1], kp, vp, o, pos, sot, slot, table_bt, status, nh, nkv, d, ps, 0,
                                   1 / math.sqrt(d))
             outs.append(o)
+            if dtype == torch.float32:          # the float32 path's own kernel: a portion in tiles, a single token in stripes
+                o = torch.empty(n, nh * d, device=dev)
+                if not ops.attention_f32(qkv, qkv.shape[1], kp, vp, o, pos, slot, mk([0, n]), table_bt, mk([0, 0]), status, int(n == 1),
+                                         int(n > 1), nh, nkv, d, ps, 0, hi, 1 / math.sqrt(d)):
+                    failures.append("float32 attention refused")
+                outs_f32.append(o)
         s64 = qkv_all.double()
 
         def norm_rope(t, wt):
@@ -96,6 +102,8 @@ def run() -> int:
         v = s64[:, (nh + nkv) * d:].view(L, nkv, d)
         want = _attention_reference(q, k, v, 1 / math.sqrt(d)).reshape(L, nh * d)
         check(f"norm+rope+cache+attention {tag}", _rel(torch.cat(outs), want), tol)
+        if outs_f32:
+            check("attention over pages, tiles and stripes f32", _rel(torch.cat(outs_f32), want), tol)
     # sampling
     logits = torch.randn(3, 5000, device=dev)
     logits[1, 77] = logits[1, 4000] = 30.0
@@ -138,7 +146,8 @@ def run() -> int:
     for name in sorted(launched):
         print(f"  {name}: {launched[name]}")
     for name in ("attention_decode_tma_kernel (merge in the cluster)", "attention_prefill_tc_kernel", "gemm_tc_pair_kernel",
-                 "gemm_tc_kernel (split-K, splits add together)", "sample_kernel"):
+                 "gemm_tc_kernel (split-K, splits add together)", "gemm_f32_kernel", "attention_f32_kernel",
+                 "attention_f32_kernel (stripes in a cluster)", "sample_kernel"):
         if launched.get(name, 0) == 0:
             failures.append(f"{name} was never launched")
     print("selftest:", "all ok" if not failures else f"FAILED: {', '.join(failures)}")

@@ -21,8 +21,10 @@ def product(a, w, mode, out=None):
     return out
 
 
-# K: below one run, one run exactly, runs with a short last one, eight runs; K = 301 and 1031 are not whole vectors
-@pytest.mark.parametrize("N,K", [(7, 5), (129, 32), (64, 301), (130, 512), (257, 1032), (66, 1031), (200, 2100)])
+# K: below one run, one run exactly, runs with a short last one, every number of runs from one to eight (clusters of that size);
+# K = 301, 1031, 1307 and 1801 are not whole vectors
+@pytest.mark.parametrize("N,K", [(7, 5), (129, 32), (64, 301), (130, 512), (70, 772), (257, 1032), (66, 1031), (130, 1284), (40, 1307),
+                                 (66, 1536), (200, 1801), (200, 2100)])
 @pytest.mark.parametrize("M", [1, 4, 5, 8, 9, 32, 33, 65])
 def test_float32_product_against_float64(M, N, K):
     from carbon_engine_b200 import ops
@@ -50,8 +52,8 @@ def test_float32_product_against_float64(M, N, K):
     assert torch.equal(product(a, w, ops.GEMM_STORE), product(aligned, w, ops.GEMM_STORE))
 
 
-# the second size has tiles enough for one block a tile from 1 token on, the first only with many tokens
-@pytest.mark.parametrize("N,K", [(1024, 2048), (38000, 520)])
+# the second size has tiles enough for one block a tile from 1 token on, the others only with many tokens
+@pytest.mark.parametrize("N,K", [(1024, 2048), (38000, 520), (1024, 800), (1024, 1300), (1024, 1536), (1024, 1800)])
 def test_float32_product_has_the_same_bits_in_every_tile_and_cluster(N, K):
     from carbon_engine_b200 import ops
     torch.manual_seed(1)

@@ -98,6 +98,19 @@ def test_products_with_few_tiles_share_k(linked):
     assert [parts(chip.gemm_tc(400, N, K, mode)) for N, K, mode in PRODUCTS[:6]] == [1, 2, 1, 2, 1, 2]
 
 
+def test_the_numbers_of_sharers_that_the_kernel_tests_run(linked):
+    from test_pair_tiles_gpu import SHARED
+    chip = Chip(linked, B200)
+    assert [parts(chip.gemm_tc(M, N, K, mode)) for M, N, K, gated, _ in SHARED for mode in ((SWIGLU, CLAMPGLU) if gated else (STORE, ACCUM))] == \
+        [n for *_, n in SHARED for _ in range(2)]
+
+
+@pytest.mark.parametrize("K,runs", [(700, 2), (800, 3), (1032, 4), (1300, 5), (1536, 6), (1800, 7), (2048, 8), (5000, 8)])
+def test_float32_products_of_few_tiles_give_each_block_of_a_cluster_a_run_of_k(linked, K, runs):
+    seen = Chip(linked, {n: 100 for n in range(2, 9)}).gemm_f32(33, 1024, K)
+    assert seen.cluster[2] == seen.grid[2] == runs
+
+
 @pytest.mark.parametrize("launch", [lambda c: c.gemm_f32(100, 4096, 4096), lambda c: c.attention_f32(0, 40), lambda c: c.gemm_tc(4, 4096, 4096),
                                     lambda c: c.gemm_tc(200, 4096, 4096), lambda c: c.gemm_tc(2048, 4096, 4096), lambda c: c.gemm_tc(2048, 128, 4096)],
                          ids=["float32 product", "float32 attention", "one-block product", "shared pairs", "pairs", "single CTAs"])
