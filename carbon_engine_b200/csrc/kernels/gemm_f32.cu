@@ -21,8 +21,9 @@
 //     8 tokens                 495 -> 28                        987 -> 28
 //     32 tokens                499 -> 60                        999 -> 51
 //     301 tokens               925 -> 448 (34 TFLOP/s)         1234 -> 234 (32 TFLOP/s)
-// At 64 tokens and more an fma.f32x2 takes three cycles of a scheduler's FMA pipe (its six operand registers come through two
-// ports), and that is the limit: the same tile with twice the warps (8 x 4 results a thread) or with scalar fmaf is 5 to 15 % slower.
+// At 301 tokens the FMA pipes are 61 % busy (an fma.f32x2 holds one for two cycles): 480 tiles on 296 places make a second wave that is
+// 0.62 full, and the two warps of a scheduler leave it without a ready one in half of the cycles.  The same tile with twice the warps
+// (8 x 4 results a thread) or with scalar fmaf is 5 to 15 % slower.
 #include "gemm_f32.cuh"
 
 namespace {

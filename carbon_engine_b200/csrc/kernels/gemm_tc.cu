@@ -923,12 +923,12 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_persistent_kernel(const __gri
 
 
 // ---------------------------------------------------------------------------------------------
-// Many tokens, CTA pairs: two CTAs of a cluster work on one tile of 256 weight rows x BN tokens with
+// Many tokens, CTA pairs: two CTAs of a cluster work on one tile of 256 weight rows x 80 to 256 tokens with
 // tcgen05.mma.cta_group::2.  Each CTA loads its own 128 weight rows and only HALF of the token tile;
 // the tensor cores of both SMs read both halves, so a pair moves a third less operand data through
 // L2 and shared memory per flop than two single CTAs (the single-CTA kernel is bound by exactly that).
-// The leader CTA's MMA thread issues the MMAs for both; it learns that the peer's stage has landed
-// from an mbarrier that the peer arrives on across the cluster; its tcgen05.commit frees the stage
+// The leader CTA's MMA warp issues the MMAs for both; it learns that a stage has landed in both from its own
+// mbarrier, on which the bytes of both are counted; its tcgen05.commit frees the stage
 // and publishes the accumulators in BOTH CTAs (commit with multicast::cluster; loads use none).
 // Each CTA runs the epilogue for its own 128 rows out of its own tensor memory.
 // ---------------------------------------------------------------------------------------------
