@@ -730,6 +730,12 @@ def gemm_plain(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, mode: int, glu
     if c.dtype != want:
         raise KernelError(f"gemm_plain: output must be {want}")
     bias, limit, alpha = glu_args(glu, mode, N)
+    if a.dtype == torch.float32 and M <= 8:
+        code = kernels().ce_gemm_f32_stream(_ptr(a), _ptr(w), _ptr(c), M, N, K, a.stride(0), c.stride(0), mode, bias, limit, alpha,
+                                            int(weights_ready), _stream())
+        if code != 1:                       # (1: sizes that the other kernel takes)
+            _ok(code)
+            return
     _ok(kernels().ce_gemm_plain(_ptr(a), _ptr(w), _ptr(c), dtype_code(a.dtype), M, N, K, a.stride(0), c.stride(0),
                                 mode, bias, limit, alpha, int(weights_ready), _stream()))
 
