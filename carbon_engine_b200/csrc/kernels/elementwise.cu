@@ -305,146 +305,72 @@ __global__ void qk_rope_kvwrite_kernel(QkRopeArgs a) {
     if (j < d) CeType<T>::store(dst + j, v);
 }
 
-// Vectors of VW consecutive elements to and from float (2 and 4 elements as one access)
-template <typename T, int VW> struct RopeVec {
-    static __device__ __forceinline__ void load(const T* p, float (&v)[VW]) {
+// Eight consecutive elements to and from float, in accesses of 16 bytes
+__device__ __forceinline__ void rope_load8(const float* p, float (&v)[8]) {
+    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void rope_load8(const __nv_bfloat16* p, float (&v)[8]) {
+    const uint4 r = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
-        for (int i = 0; i < VW; ++i) v[i] = CeType<T>::load(p + i);
-    }
-    static __device__ __forceinline__ void store(T* p, const float (&v)[VW]) {
-#pragma unroll
-        for (int i = 0; i < VW; ++i) CeType<T>::store(p + i, v[i]);
-    }
-};
-template <> struct RopeVec<float, 2> {
-    static __device__ __forceinline__ void load(const float* p, float (&v)[2]) { float2 t = *reinterpret_cast<const float2*>(p); v[0] = t.x; v[1] = t.y; }
-    static __device__ __forceinline__ void store(float* p, const float (&v)[2]) { *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]); }
-};
-template <> struct RopeVec<float, 4> {
-    static __device__ __forceinline__ void load(const float* p, float (&v)[4]) { float4 t = *reinterpret_cast<const float4*>(p); v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w; }
-    static __device__ __forceinline__ void store(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
-};
-template <> struct RopeVec<__nv_bfloat16, 2> {
-    static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&v)[2]) {
-        float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); v[0] = t.x; v[1] = t.y;
-    }
-    static __device__ __forceinline__ void store(__nv_bfloat16* p, const float (&v)[2]) {
-        *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(v[0], v[1]);
-    }
-};
-template <> struct RopeVec<__nv_bfloat16, 4> {
-    static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&v)[4]) {
-        uint2 r = *reinterpret_cast<const uint2*>(p);
-        float2 lo = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&r.x)), hi = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&r.y));
-        v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
-    }
-    static __device__ __forceinline__ void store(__nv_bfloat16* p, const float (&v)[4]) {
-        __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
-        uint2 r;
-        r.x = *reinterpret_cast<uint32_t*>(&lo); r.y = *reinterpret_cast<uint32_t*>(&hi);
-        *reinterpret_cast<uint2*>(p) = r;
-    }
-};
-
-// Head sizes that are multiples of 64 (up to 256) with a full rotation: one warp per group of `hpw`
-// consecutive heads of one token.  A lane holds VW = d/64 consecutive elements of the first half of a
-// head and the VW elements d/2 further on, their partners in the rotation, so nothing is exchanged
-// between lanes but the sum of squares.  The token's position, page, cosines and sines are looked up
-// once per warp, a head's address is the last one plus a stride, and the elements of four heads are in
-// flight together; with one head per warp (few tokens: decoding) the grid is as large as it can be, with many (portions of
-// prompts) a token's heads share the lookups.  A head's arithmetic does not depend on hpw.
-// n heads, one after the other from src (stride d) to dst (stride dst_stride): RMS norm with weights w1/w2
-// (NORM), rotation by cs/sn (ROT), or neither (values: a copy).  Four heads are in flight together.
-template <typename T, int VW, bool NORM, bool ROT>
-__device__ __forceinline__ void rope_heads(const T* src, T* dst, size_t dst_stride, int n, int d, int e0, float eps,
-                                           const float (&w1)[VW], const float (&w2)[VW], const float (&cs)[VW],
-                                           const float (&sn)[VW]) {
-    constexpr int U = 4;
-    int half = d >> 1;
-    float inv_d = 1.0f / (float)d;
-    for (int hb = 0; hb < n; hb += U) {
-        float x1[U][VW], x2[U][VW];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (hb + u < n) {
-                RopeVec<T, VW>::load(src + (size_t)u * d + e0, x1[u]);
-                RopeVec<T, VW>::load(src + (size_t)u * d + half + e0, x2[u]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (hb + u >= n) break;
-            if (NORM) {
-                float ss = 0.f;
-#pragma unroll
-                for (int i = 0; i < VW; ++i) ss = fmaf(x1[u][i], x1[u][i], ss);
-#pragma unroll
-                for (int i = 0; i < VW; ++i) ss = fmaf(x2[u][i], x2[u][i], ss);
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-                float inv = rsqrtf(fmaf(ss, inv_d, eps));
-#pragma unroll
-                for (int i = 0; i < VW; ++i) { x1[u][i] = x1[u][i] * inv * w1[i]; x2[u][i] = x2[u][i] * inv * w2[i]; }
-            }
-            if (ROT) {
-#pragma unroll
-                for (int i = 0; i < VW; ++i) {
-                    float p = x1[u][i], q = x2[u][i];
-                    x1[u][i] = p * cs[i] - q * sn[i];
-                    x2[u][i] = q * cs[i] + p * sn[i];
-                }
-            }
-            RopeVec<T, VW>::store(dst + u * dst_stride + e0, x1[u]);
-            RopeVec<T, VW>::store(dst + u * dst_stride + half + e0, x2[u]);
-        }
-        src += (size_t)U * d;
-        dst += U * dst_stride;
+    for (int i = 0; i < 4; ++i) {
+        const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+        v[2 * i] = t.x; v[2 * i + 1] = t.y;
     }
 }
-
-template <typename T, int VW>
-__device__ __forceinline__ void rope_heads_any(const T* src, T* dst, size_t dst_stride, int n, int d, int e0, float eps,
-                                               const float* w, bool rot, const float (&cs)[VW], const float (&sn)[VW]) {
-    float w1[VW], w2[VW];
+__device__ __forceinline__ void rope_store8(float* p, const float (&v)[8]) {
+    reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ void rope_store8(__nv_bfloat16* p, const float (&v)[8]) {
+    uint32_t w[4];
 #pragma unroll
-    for (int i = 0; i < VW; ++i) w1[i] = w2[i] = 1.f;
-    if (w) {
-        RopeVec<float, VW>::load(w + e0, w1);
-        RopeVec<float, VW>::load(w + (d >> 1) + e0, w2);
+    for (int i = 0; i < 4; ++i) {
+        const __nv_bfloat162 t = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+        w[i] = *reinterpret_cast<const uint32_t*>(&t);
     }
-    if (w && rot) rope_heads<T, VW, true, true>(src, dst, dst_stride, n, d, e0, eps, w1, w2, cs, sn);
-    else if (w) rope_heads<T, VW, true, false>(src, dst, dst_stride, n, d, e0, eps, w1, w2, cs, sn);
-    else if (rot) rope_heads<T, VW, false, true>(src, dst, dst_stride, n, d, e0, eps, w1, w2, cs, sn);
-    else rope_heads<T, VW, false, false>(src, dst, dst_stride, n, d, e0, eps, w1, w2, cs, sn);
+    *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-template <typename T, int VW>
+// Head sizes that are multiples of 64 (up to 256) with a full rotation.  A head belongs to L neighbouring lanes (the power of two from
+// d / 16 on; with heads of 192 four of sixteen idle): a lane holds 8 consecutive elements of the head's first half and the 8 elements
+// d/2 further on, their partners in the rotation, so every access is 16 bytes, a warp takes 32 / L heads at a time, and nothing is
+// exchanged between lanes but the sum of squares.  The token's position, page, cosines and sines are looked up once per warp; a warp
+// takes `hpw` consecutive heads of one token, as few as it takes at a time where tokens are few (decoding: as large a grid as can be),
+// a quarter of them all in portions of prompts.  A head's arithmetic does not depend on hpw.
+// What bounds a long portion is the memory (2,048 tokens of 32 + 2 x 8 heads of 128: 50 MB in and out); with accesses of 4 bytes a lane it
+// was the instructions.  Measured: a prompt of 203 tokens, 12 layers of 8b sizes, 2,306 -> 2,243 us a pass; eight decode steps with this and
+// the attention's merge in one trip 10,330 -> 10,040 (one request), 11,440 -> 11,152 (eight).
+template <typename T, int L>
 __global__ void __launch_bounds__(128) qk_rope_kvwrite_warp_kernel(QkRopeArgs a, int hpw) {
     // positions, slots, block tables, cosines, sines and norm weights are inputs of the step or constants:
     // they are looked up while the kernel before this one (the QKV product) still runs; only its output waits
     ce_pdl_launch_dependents();
-    int lane = threadIdx.x & 31;
-    int heads_per_token = a.nh + 2 * a.nkv;
-    int groups = (heads_per_token + hpw - 1) / hpw;
-    long long wg = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    constexpr int AT_ONCE = 32 / L;
+    const int lane = threadIdx.x & 31, sub = lane / L, heads_per_token = a.nh + 2 * a.nkv;
+    const int groups = (heads_per_token + hpw - 1) / hpw;
+    const long long wg = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
     if (wg >= (long long)a.T * groups) return;
-    int t = (int)(wg / groups), g = (int)(wg - (long long)t * groups);
-    int hh0 = g * hpw, hh1 = min(hh0 + hpw, heads_per_token);
+    const int t = (int)(wg / groups), g = (int)(wg - (long long)t * groups);
+    const int hh0 = g * hpw;
+    int hh1 = min(hh0 + hpw, heads_per_token);
     if (!a.write_kv) hh1 = min(hh1, a.nh);
     if (hh0 >= hh1) return;
-    int d = a.d, half = d >> 1, e0 = VW * lane;
-    int pos = a.positions[t];
-    bool rotate = a.cos_table != nullptr;
+    const int d = a.d, half = d >> 1, e0 = 8 * (lane % L);
+    const bool mine = e0 < half;
+    const int pos = a.positions[t];
+    const bool rotate = a.cos_table != nullptr;
     if (rotate && pos >= a.max_pos && hh0 < a.nh + a.nkv) {
         if (lane == 0) atomicExch(a.status, 3);
         return;
     }
-    float cs[VW], sn[VW];
+    float cs[8], sn[8];
 #pragma unroll
-    for (int i = 0; i < VW; ++i) { cs[i] = 1.f; sn[i] = 0.f; }
-    if (rotate && hh0 < a.nh + a.nkv) {
-        RopeVec<float, VW>::load(a.cos_table + (size_t)pos * half + e0, cs);
-        RopeVec<float, VW>::load(a.sin_table + (size_t)pos * half + e0, sn);
+    for (int i = 0; i < 8; ++i) { cs[i] = 1.f; sn[i] = 0.f; }
+    if (rotate && mine && hh0 < a.nh + a.nkv) {
+        rope_load8(a.cos_table + (size_t)pos * half + e0, cs);
+        rope_load8(a.sin_table + (size_t)pos * half + e0, sn);
     }
     size_t page_row = 0;
     if (hh1 > a.nh) {                      // a K or V head in this group: where the token's row lies in the pools
@@ -457,36 +383,84 @@ __global__ void __launch_bounds__(128) qk_rope_kvwrite_warp_kernel(QkRopeArgs a,
         page_row = (size_t)page * a.nkv * a.page_size + pos % a.page_size;
     }
     T* row = (T*)a.qkv + (size_t)t * heads_per_token * d;
+    const float inv_d = 1.0f / (float)d;
+    float w1[8], w2[8];
+    const float* held = nullptr;           // the norm weights in w1 and w2
+    auto hold = [&](const float* w) {
+        if (!w || w == held || !mine) return;
+        rope_load8(w + e0, w1);
+        rope_load8(w + half + e0, w2);
+        held = w;
+    };
+    auto weights_of = [&](int hh) { return hh < a.nh ? a.q_weight : hh < a.nh + a.nkv ? a.k_weight : nullptr; };
+    hold(weights_of(hh0 + sub));
     ce_pdl_wait();
-    // the group's query heads (in place), key heads and value heads (into the pools)
-    int q1 = min(hh1, a.nh);
-    if (hh0 < q1) rope_heads_any<T, VW>(row + (size_t)hh0 * d, row + (size_t)hh0 * d, (size_t)d, q1 - hh0, d, e0, a.eps, a.q_weight, rotate, cs, sn);
-    int k0 = max(hh0, a.nh), k1 = min(hh1, a.nh + a.nkv);
-    if (k0 < k1)
-        rope_heads_any<T, VW>(row + (size_t)k0 * d, (T*)a.k_pool + (page_row + (size_t)(k0 - a.nh) * a.page_size) * d,
-                              (size_t)a.page_size * d, k1 - k0, d, e0, a.eps, a.k_weight, rotate, cs, sn);
-    int v0 = max(hh0, a.nh + a.nkv);
-    if (v0 < hh1)
-        rope_heads_any<T, VW>(row + (size_t)v0 * d, (T*)a.v_pool + (page_row + (size_t)(v0 - a.nh - a.nkv) * a.page_size) * d,
-                              (size_t)a.page_size * d, hh1 - v0, d, e0, a.eps, nullptr, false, cs, sn);
+    constexpr int U = 2;                   // heads of a lane in flight together
+    for (int hb = hh0; hb < hh1; hb += U * AT_ONCE) {
+        float x1[U][8], x2[U][8];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int hh = hb + u * AT_ONCE + sub;
+            if (hh < hh1 && mine) {
+                rope_load8(row + (size_t)hh * d + e0, x1[u]);
+                rope_load8(row + (size_t)hh * d + half + e0, x2[u]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) x1[u][i] = x2[u][i] = 0.f;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (hb + u * AT_ONCE >= hh1) break;
+            // query heads stay in place, key and value heads go into the pools; values are copied as they are
+            const int hh = hb + u * AT_ONCE + sub, kv = hh - a.nh, v = kv - a.nkv;
+            const float* w = weights_of(hh);
+            hold(w);
+            float ss = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ss = fmaf(x1[u][i], x1[u][i], ss);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ss = fmaf(x2[u][i], x2[u][i], ss);
+#pragma unroll
+            for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if (hh >= hh1 || !mine) continue;
+            T* dst = kv < 0 ? row + (size_t)hh * d : (T*)(v < 0 ? a.k_pool : a.v_pool) + (page_row + (size_t)(v < 0 ? kv : v) * a.page_size) * d;
+            if (w) {
+                const float inv = rsqrtf(fmaf(ss, inv_d, a.eps));
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { x1[u][i] = x1[u][i] * inv * w1[i]; x2[u][i] = x2[u][i] * inv * w2[i]; }
+            }
+            if (rotate && v < 0) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float p = x1[u][i], q = x2[u][i];
+                    x1[u][i] = p * cs[i] - q * sn[i];
+                    x2[u][i] = q * cs[i] + p * sn[i];
+                }
+            }
+            rope_store8(dst + e0, x1[u]);
+            rope_store8(dst + half + e0, x2[u]);
+        }
+    }
 }
 
 template <typename T>
 static bool launch_rope_warp(const QkRopeArgs& a, cudaStream_t stream) {
-    int heads_per_token = a.nh + 2 * a.nkv;
+    const int heads_per_token = a.nh + 2 * a.nkv;
     if (a.d % 64 || a.d > 256 || (a.cos_table && (a.rd != a.d || a.pairing != 0))) return false;
-    // few tokens: a warp per head; many: four warps share a token's heads
-    int hpw = a.T >= 256 ? (heads_per_token + 3) / 4 : 1;
-    long long warps = (long long)a.T * ((heads_per_token + hpw - 1) / hpw);
+    if (((uintptr_t)a.qkv | (uintptr_t)a.k_pool | (uintptr_t)a.v_pool | (uintptr_t)a.q_weight | (uintptr_t)a.k_weight |
+         (uintptr_t)a.cos_table | (uintptr_t)a.sin_table) & 15) return false;                 // (accesses of 16 bytes)
+    const int lanes = a.d <= 64 ? 4 : a.d <= 128 ? 8 : 16, at_once = 32 / lanes;
+    // few tokens: as many warps as there are; many: four warps share a token's heads
+    const int hpw = a.T >= 256 ? ((heads_per_token + 3) / 4 + at_once - 1) / at_once * at_once : at_once;
+    const long long warps = (long long)a.T * ((heads_per_token + hpw - 1) / hpw);
     if ((warps + 3) / 4 > 2147483647LL) return false;
-    unsigned blocks = (unsigned)((warps + 3) / 4);
-    switch (a.d / 64) {
-        case 1: { ce_note("qk_rope_kvwrite_warp_kernel"); ce_launch(qk_rope_kvwrite_warp_kernel<T, 1>, blocks, 128, 0, stream, a, hpw); } return true;
-        case 2: { ce_note("qk_rope_kvwrite_warp_kernel"); ce_launch(qk_rope_kvwrite_warp_kernel<T, 2>, blocks, 128, 0, stream, a, hpw); } return true;
-        case 3: { ce_note("qk_rope_kvwrite_warp_kernel"); ce_launch(qk_rope_kvwrite_warp_kernel<T, 3>, blocks, 128, 0, stream, a, hpw); } return true;
-        case 4: { ce_note("qk_rope_kvwrite_warp_kernel"); ce_launch(qk_rope_kvwrite_warp_kernel<T, 4>, blocks, 128, 0, stream, a, hpw); } return true;
-    }
-    return false;
+    const unsigned blocks = (unsigned)((warps + 3) / 4);
+    ce_note("qk_rope_kvwrite_warp_kernel");
+    if (lanes == 4) ce_launch(qk_rope_kvwrite_warp_kernel<T, 4>, blocks, 128, 0, stream, a, hpw);
+    else if (lanes == 8) ce_launch(qk_rope_kvwrite_warp_kernel<T, 8>, blocks, 128, 0, stream, a, hpw);
+    else ce_launch(qk_rope_kvwrite_warp_kernel<T, 16>, blocks, 128, 0, stream, a, hpw);
+    return true;
 }
 
 extern "C" int ce_qk_rope_kvwrite(void* qkv, void* k_pool, void* v_pool, int dtype, const float* q_weight,
