@@ -56,14 +56,21 @@ class StepBuffers:
         else:
             self.status = torch.zeros(1, dtype=torch.int32, device=device)
         self._uploaded = None
+        self._views = {}
 
     def host_section(self, name: str) -> np.ndarray:
         off, n = self.offsets[name]
         return self.host_np[off:off + n]
 
     def dev_section(self, name: str, n: Optional[int] = None) -> torch.Tensor:
-        off, cap = self.offsets[name]
-        return self.dev[off:off + (cap if n is None else n)]
+        # a step asks for a dozen views of the same buffer, most of them as the step before it did
+        view = self._views.get((name, n))
+        if view is None:
+            if len(self._views) >= 512:
+                self._views.clear()
+            off, cap = self.offsets[name]
+            view = self._views[(name, n)] = self.dev[off:off + (cap if n is None else n)]
+        return view
 
     def wait_host_free(self) -> None:
         """Block until the last upload has left the pinned buffer, so that it may be rewritten."""

@@ -50,6 +50,9 @@ class Scheduler:
         self.max_step_tokens = max(max_step_tokens, self.max_running)
         self._entries = np.zeros(5 * (self.max_running + 1), dtype=np.int64)
         self._tokens = np.zeros(self.max_step_tokens + 1, dtype=np.int32)
+        # (numpy makes a ctypes pointer in microseconds: those of the kept arrays are made once)
+        self._p_entries = self._entries.ctypes.data_as(ctypes.POINTER(ctypes.c_int64))
+        self._p_tokens = self._tokens.ctypes.data_as(ctypes.POINTER(ctypes.c_int32))
         self._fin = None                     # buffers of pop_finished, made at its first call
 
     def __del__(self):
@@ -69,20 +72,17 @@ class Scheduler:
 
     def plan(self) -> List[PlanEntry]:
         n_tok = ctypes.c_int(0)
-        n = self._lib.sched_plan(self._h, self._entries.ctypes.data_as(ctypes.POINTER(ctypes.c_int64)),
-                                 len(self._entries) // 5, self._tokens.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)),
-                                 len(self._tokens), ctypes.byref(n_tok))
+        n = self._lib.sched_plan(self._h, self._p_entries, len(self._entries) // 5, self._p_tokens, len(self._tokens),
+                                 ctypes.byref(n_tok))
         return self._read_plan(n, n_tok.value)
 
     def plan_for(self, request_ids: Sequence[int]) -> List[PlanEntry]:
         """The step that is already on the device for ``request_ids`` (one token each, fed there from the last
         step's picks): its entries for those of them that still run.  Nothing is admitted."""
-        ids = np.ascontiguousarray(request_ids, dtype=np.int64)
+        n_ids = len(request_ids)
         n_tok = ctypes.c_int(0)
-        n = self._lib.sched_plan_for(self._h, ids.ctypes.data_as(ctypes.POINTER(ctypes.c_int64)), len(ids),
-                                     self._entries.ctypes.data_as(ctypes.POINTER(ctypes.c_int64)), len(self._entries) // 5,
-                                     self._tokens.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), len(self._tokens),
-                                     ctypes.byref(n_tok))
+        n = self._lib.sched_plan_for(self._h, (ctypes.c_int64 * n_ids)(*request_ids), n_ids, self._p_entries, len(self._entries) // 5,
+                                     self._p_tokens, len(self._tokens), ctypes.byref(n_tok))
         return self._read_plan(n, n_tok.value)
 
     def _read_plan(self, n: int, n_tok: int) -> List[PlanEntry]:
@@ -109,8 +109,8 @@ class Scheduler:
         return self._lib.sched_running(self._h)
 
     def commit(self, sampled: Sequence[int]) -> None:
-        s = np.ascontiguousarray(sampled, dtype=np.int32)
-        if self._lib.sched_commit(self._h, s.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), len(s)) != 0:
+        n = len(sampled)
+        if self._lib.sched_commit(self._h, (ctypes.c_int32 * n)(*sampled), n) != 0:
             raise RuntimeError("commit: the number of sampled tokens does not match the plan")
 
     def fail_step(self) -> None:
