@@ -305,49 +305,46 @@ __global__ void qk_rope_kvwrite_kernel(QkRopeArgs a) {
     if (j < d) CeType<T>::store(dst + j, v);
 }
 
-// Eight consecutive elements to and from float, in accesses of 16 bytes
-__device__ __forceinline__ void rope_load8(const float* p, float (&v)[8]) {
-    const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-}
-__device__ __forceinline__ void rope_load8(const __nv_bfloat16* p, float (&v)[8]) {
-    const uint4 r = *reinterpret_cast<const uint4*>(p);
-    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+// E consecutive elements to and from float, W of them an access
+template <typename T, int W> struct alignas(W * sizeof(T)) RopePiece { T e[W]; };
+template <int W, typename T, int E>
+__device__ __forceinline__ void rope_load(const T* p, float (&v)[E]) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float2 t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
-        v[2 * i] = t.x; v[2 * i + 1] = t.y;
+    for (int i = 0; i < E; i += W) {
+        const RopePiece<T, W> piece = *reinterpret_cast<const RopePiece<T, W>*>(p + i);
+#pragma unroll
+        for (int j = 0; j < W; ++j) v[i + j] = CeType<T>::load(piece.e + j);
     }
 }
-__device__ __forceinline__ void rope_store8(float* p, const float (&v)[8]) {
-    reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
-    reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
-}
-__device__ __forceinline__ void rope_store8(__nv_bfloat16* p, const float (&v)[8]) {
-    uint32_t w[4];
+template <int W, typename T, int E>
+__device__ __forceinline__ void rope_store(T* p, const float (&v)[E]) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const __nv_bfloat162 t = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-        w[i] = *reinterpret_cast<const uint32_t*>(&t);
+    for (int i = 0; i < E; i += W) {
+        RopePiece<T, W> piece;
+#pragma unroll
+        for (int j = 0; j < W; ++j) CeType<T>::store(piece.e + j, v[i + j]);
+        *reinterpret_cast<RopePiece<T, W>*>(p + i) = piece;
     }
-    *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// Head sizes that are multiples of 64 (up to 256) with a full rotation.  A head belongs to L neighbouring lanes (the power of two from
-// d / 16 on; with heads of 192 four of sixteen idle): a lane holds 8 consecutive elements of the head's first half and the 8 elements
-// d/2 further on, their partners in the rotation, so every access is 16 bytes, a warp takes 32 / L heads at a time, and nothing is
+// Head sizes that are multiples of 64 (up to 256) with a full rotation.  A head belongs to L neighbouring lanes: a lane holds E
+// consecutive elements of the head's first half and the E elements d/2 further on, their partners in the rotation (E = 8, so accesses
+// of 16 bytes; heads of 192 take E = 12, which bfloat16 reads 8 bytes at a time), a warp takes 32 / L heads at a time, and nothing is
 // exchanged between lanes but the sum of squares.  The token's position, page, cosines and sines are looked up once per warp; a warp
 // takes `hpw` consecutive heads of one token, as few as it takes at a time where tokens are few (decoding: as large a grid as can be),
 // a quarter of them all in portions of prompts.  A head's arithmetic does not depend on hpw.
+// The sum of squares is that of a warp of 32 lanes with d/64 elements of each half: such a lane's terms in order, first half then
+// second, and the lanes' sums by halves (lanes 16 apart, 8, 4, 2, 1).  A lane here holds 32 / L of those lanes' sums.
 // What bounds a long portion is the memory (2,048 tokens of 32 + 2 x 8 heads of 128: 50 MB in and out); with accesses of 4 bytes a lane it
 // was the instructions.  Measured: a prompt of 203 tokens, 12 layers of 8b sizes, 2,306 -> 2,243 us a pass; eight decode steps with this and
 // the attention's merge in one trip 10,330 -> 10,040 (one request), 11,440 -> 11,152 (eight).
-template <typename T, int L>
+template <typename T, int E, int L>
 __global__ void __launch_bounds__(128) qk_rope_kvwrite_warp_kernel(QkRopeArgs a, int hpw) {
     // positions, slots, block tables, cosines, sines and norm weights are inputs of the step or constants:
     // they are looked up while the kernel before this one (the QKV product) still runs; only its output waits
     ce_pdl_launch_dependents();
-    constexpr int AT_ONCE = 32 / L;
+    constexpr int AT_ONCE = 32 / L, SUMS = 32 / L, TERMS = E / SUMS;
+    constexpr int W = E * sizeof(T) % 16 ? 8 / sizeof(T) : 16 / sizeof(T);
     const int lane = threadIdx.x & 31, sub = lane / L, heads_per_token = a.nh + 2 * a.nkv;
     const int groups = (heads_per_token + hpw - 1) / hpw;
     const long long wg = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -357,20 +354,20 @@ __global__ void __launch_bounds__(128) qk_rope_kvwrite_warp_kernel(QkRopeArgs a,
     int hh1 = min(hh0 + hpw, heads_per_token);
     if (!a.write_kv) hh1 = min(hh1, a.nh);
     if (hh0 >= hh1) return;
-    const int d = a.d, half = d >> 1, e0 = 8 * (lane % L);
-    const bool mine = e0 < half;
+    constexpr int half = E * L, d = 2 * half;
+    const int e0 = E * (lane % L);
     const int pos = a.positions[t];
     const bool rotate = a.cos_table != nullptr;
     if (rotate && pos >= a.max_pos && hh0 < a.nh + a.nkv) {
         if (lane == 0) atomicExch(a.status, 3);
         return;
     }
-    float cs[8], sn[8];
+    float cs[E], sn[E];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { cs[i] = 1.f; sn[i] = 0.f; }
-    if (rotate && mine && hh0 < a.nh + a.nkv) {
-        rope_load8(a.cos_table + (size_t)pos * half + e0, cs);
-        rope_load8(a.sin_table + (size_t)pos * half + e0, sn);
+    for (int i = 0; i < E; ++i) { cs[i] = 1.f; sn[i] = 0.f; }
+    if (rotate && hh0 < a.nh + a.nkv) {
+        rope_load<4>(a.cos_table + (size_t)pos * half + e0, cs);
+        rope_load<4>(a.sin_table + (size_t)pos * half + e0, sn);
     }
     size_t page_row = 0;
     if (hh1 > a.nh) {                      // a K or V head in this group: where the token's row lies in the pools
@@ -384,12 +381,12 @@ __global__ void __launch_bounds__(128) qk_rope_kvwrite_warp_kernel(QkRopeArgs a,
     }
     T* row = (T*)a.qkv + (size_t)t * heads_per_token * d;
     const float inv_d = 1.0f / (float)d;
-    float w1[8], w2[8];
+    float w1[E], w2[E];
     const float* held = nullptr;           // the norm weights in w1 and w2
     auto hold = [&](const float* w) {
-        if (!w || w == held || !mine) return;
-        rope_load8(w + e0, w1);
-        rope_load8(w + half + e0, w2);
+        if (!w || w == held) return;
+        rope_load<4>(w + e0, w1);
+        rope_load<4>(w + half + e0, w2);
         held = w;
     };
     auto weights_of = [&](int hh) { return hh < a.nh ? a.q_weight : hh < a.nh + a.nkv ? a.k_weight : nullptr; };
@@ -397,16 +394,16 @@ __global__ void __launch_bounds__(128) qk_rope_kvwrite_warp_kernel(QkRopeArgs a,
     ce_pdl_wait();
     constexpr int U = 2;                   // heads of a lane in flight together
     for (int hb = hh0; hb < hh1; hb += U * AT_ONCE) {
-        float x1[U][8], x2[U][8];
+        float x1[U][E], x2[U][E];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int hh = hb + u * AT_ONCE + sub;
-            if (hh < hh1 && mine) {
-                rope_load8(row + (size_t)hh * d + e0, x1[u]);
-                rope_load8(row + (size_t)hh * d + half + e0, x2[u]);
+            if (hh < hh1) {
+                rope_load<W>(row + (size_t)hh * d + e0, x1[u]);
+                rope_load<W>(row + (size_t)hh * d + half + e0, x2[u]);
             } else {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) x1[u][i] = x2[u][i] = 0.f;
+                for (int i = 0; i < E; ++i) x1[u][i] = x2[u][i] = 0.f;
             }
         }
 #pragma unroll
@@ -416,30 +413,40 @@ __global__ void __launch_bounds__(128) qk_rope_kvwrite_warp_kernel(QkRopeArgs a,
             const int hh = hb + u * AT_ONCE + sub, kv = hh - a.nh, v = kv - a.nkv;
             const float* w = weights_of(hh);
             hold(w);
-            float ss = 0.f;
+            float ss[SUMS];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) ss = fmaf(x1[u][i], x1[u][i], ss);
+            for (int g = 0; g < SUMS; ++g) {
+                ss[g] = 0.f;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) ss = fmaf(x2[u][i], x2[u][i], ss);
+                for (int i = g * TERMS; i < (g + 1) * TERMS; ++i) ss[g] = fmaf(x1[u][i], x1[u][i], ss[g]);
 #pragma unroll
-            for (int o = L / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-            if (hh >= hh1 || !mine) continue;
+                for (int i = g * TERMS; i < (g + 1) * TERMS; ++i) ss[g] = fmaf(x2[u][i], x2[u][i], ss[g]);
+            }
+#pragma unroll
+            for (int o = L / 2; o > 0; o >>= 1)
+#pragma unroll
+                for (int g = 0; g < SUMS; ++g) ss[g] += __shfl_xor_sync(0xffffffffu, ss[g], o);
+#pragma unroll
+            for (int o = SUMS / 2; o > 0; o >>= 1)
+#pragma unroll
+                for (int g = 0; g < o; ++g) ss[g] += ss[g + o];
+            if (hh >= hh1) continue;
             T* dst = kv < 0 ? row + (size_t)hh * d : (T*)(v < 0 ? a.k_pool : a.v_pool) + (page_row + (size_t)(v < 0 ? kv : v) * a.page_size) * d;
             if (w) {
-                const float inv = rsqrtf(fmaf(ss, inv_d, a.eps));
+                const float inv = rsqrtf(fmaf(ss[0], inv_d, a.eps));
 #pragma unroll
-                for (int i = 0; i < 8; ++i) { x1[u][i] = x1[u][i] * inv * w1[i]; x2[u][i] = x2[u][i] * inv * w2[i]; }
+                for (int i = 0; i < E; ++i) { x1[u][i] = x1[u][i] * inv * w1[i]; x2[u][i] = x2[u][i] * inv * w2[i]; }
             }
             if (rotate && v < 0) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < E; ++i) {
                     const float p = x1[u][i], q = x2[u][i];
                     x1[u][i] = p * cs[i] - q * sn[i];
                     x2[u][i] = q * cs[i] + p * sn[i];
                 }
             }
-            rope_store8(dst + e0, x1[u]);
-            rope_store8(dst + half + e0, x2[u]);
+            rope_store<W>(dst + e0, x1[u]);
+            rope_store<W>(dst + half + e0, x2[u]);
         }
     }
 }
@@ -450,16 +457,19 @@ static bool launch_rope_warp(const QkRopeArgs& a, cudaStream_t stream) {
     if (a.d % 64 || a.d > 256 || (a.cos_table && (a.rd != a.d || a.pairing != 0))) return false;
     if (((uintptr_t)a.qkv | (uintptr_t)a.k_pool | (uintptr_t)a.v_pool | (uintptr_t)a.q_weight | (uintptr_t)a.k_weight |
          (uintptr_t)a.cos_table | (uintptr_t)a.sin_table) & 15) return false;                 // (accesses of 16 bytes)
-    const int lanes = a.d <= 64 ? 4 : a.d <= 128 ? 8 : 16, at_once = 32 / lanes;
+    const int lanes = a.d == 64 ? 4 : a.d == 256 ? 16 : 8, at_once = 32 / lanes;
     // few tokens: as many warps as there are; many: four warps share a token's heads
     const int hpw = a.T >= 256 ? ((heads_per_token + 3) / 4 + at_once - 1) / at_once * at_once : at_once;
     const long long warps = (long long)a.T * ((heads_per_token + hpw - 1) / hpw);
     if ((warps + 3) / 4 > 2147483647LL) return false;
     const unsigned blocks = (unsigned)((warps + 3) / 4);
     ce_note("qk_rope_kvwrite_warp_kernel");
-    if (lanes == 4) ce_launch(qk_rope_kvwrite_warp_kernel<T, 4>, blocks, 128, 0, stream, a, hpw);
-    else if (lanes == 8) ce_launch(qk_rope_kvwrite_warp_kernel<T, 8>, blocks, 128, 0, stream, a, hpw);
-    else ce_launch(qk_rope_kvwrite_warp_kernel<T, 16>, blocks, 128, 0, stream, a, hpw);
+    switch (a.d) {
+        case 64: ce_launch(qk_rope_kvwrite_warp_kernel<T, 8, 4>, blocks, 128, 0, stream, a, hpw); break;
+        case 128: ce_launch(qk_rope_kvwrite_warp_kernel<T, 8, 8>, blocks, 128, 0, stream, a, hpw); break;
+        case 192: ce_launch(qk_rope_kvwrite_warp_kernel<T, 12, 8>, blocks, 128, 0, stream, a, hpw); break;
+        default: ce_launch(qk_rope_kvwrite_warp_kernel<T, 8, 16>, blocks, 128, 0, stream, a, hpw); break;
+    }
     return true;
 }
 

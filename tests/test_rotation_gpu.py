@@ -1,0 +1,55 @@
+"""The rotation's warp kernel (head sizes 64 to 256, full rotation in half pairs): the order of its sums, and its walk over a token's heads."""
+import pytest
+import torch
+
+from test_kernels_gpu import DTYPES, dev, paged_layout, status, step_meta
+
+pytestmark = pytest.mark.gpu
+NAME = "qk_rope_kvwrite_warp_kernel"
+EPS = 1e-5
+
+
+def add_square(sums, x):
+    """fma(x, x, sums) of float32 values."""
+    return (x.double() * x.double() + sums.double()).float()
+
+
+def rms_norm(x, weight):
+    """The norm as a warp of 32 lanes takes it that hold d / 64 elements of each half: bit for bit."""
+    x = x.float()
+    d = x.shape[-1]
+    halves = x.reshape(*x.shape[:-1], 2, 32, d // 64)
+    sums = torch.zeros(halves.shape[:-3] + (32,), device=x.device)
+    for h in range(2):
+        for i in range(d // 64):
+            sums = add_square(sums, halves[..., h, :, i])
+    lane = torch.arange(32, device=x.device)
+    for o in (16, 8, 4, 2, 1):
+        sums = sums + sums[..., lane ^ o]
+    mean = (sums[..., :1].double() * torch.tensor(1.0 / d, dtype=torch.float32).item() + torch.tensor(EPS, dtype=torch.float32).item()).float()
+    return x * torch.rsqrt(mean) * weight
+
+
+def pool_rows(pool, table, positions, page_size):
+    """[T, nkv, d]: where the tokens of sequence 0 lie."""
+    pos = positions.long()
+    return pool[table[0].long()[pos // page_size], :, pos % page_size, :]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("nh,nkv,d", [(5, 3, 64), (6, 2, 128), (7, 1, 192), (5, 2, 256)])
+@pytest.mark.parametrize("T", [3, 260])
+def test_the_norm_keeps_the_order_of_its_sums(dtype, nh, nkv, d, T):
+    from carbon_engine_b200 import ops
+    torch.manual_seed(d + T)
+    table, kp, vp = paged_layout([T], 16, nkv, d, dtype)
+    qkv = (torch.randn(T, (nh + 2 * nkv) * d, device=dev()) * 3).to(dtype)
+    qw, kw = 1 + 0.2 * torch.randn(d, device=dev()), 1 + 0.2 * torch.randn(d, device=dev())
+    positions, sot, slots = step_meta([(0, T)])
+    heads = qkv.view(T, nh + 2 * nkv, d).clone()
+    before, st = ops.kernel_counts().get(NAME, 0), status()
+    ops.qk_rope_kvwrite(qkv, kp, vp, qw, kw, None, None, positions, sot, slots, table, st, nh, nkv, d, 0, 16, EPS)
+    assert ops.kernel_counts().get(NAME, 0) == before + 1 and st.item() == 0
+    assert torch.equal(qkv.view(T, nh + 2 * nkv, d)[:, :nh], rms_norm(heads[:, :nh], qw).to(dtype))
+    assert torch.equal(pool_rows(kp, table, positions, 16), rms_norm(heads[:, nh:nh + nkv], kw).to(dtype))
+    assert torch.equal(pool_rows(vp, table, positions, 16), heads[:, nh + nkv:])
