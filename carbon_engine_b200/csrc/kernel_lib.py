@@ -28,9 +28,9 @@ _SIGNATURES = {
     # x, w, out, out_dtype, rows, R, H, eps, stream
     "ce_rmsnorm": (_i, [_p, _p, _p, _i, _p, _i, _i, _f, _p]),
     # qkv, k_pool, v_pool, dtype, qw, kw, cos, sin, positions, seq_of_token, seq_slot, block_table, status,
-    # T, nh, nkv, d, rd, page_size, max_pages, num_pages, max_pos, write_kv, eps, pairing, stream
+    # T, nh, nkv, d, rd, page_size, max_pages, num_pages, max_pos, write_kv, eps, pairing, weights_ready, stream
     "ce_qk_rope_kvwrite": (_i, [_p, _p, _p, _i, _p, _p, _p, _p, _p, _p, _p, _p, _p,
-                                _i, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _p]),
+                                _i, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _i, _p]),
     "ce_add_residual": (_i, [_p, _p, _i, _ll, _p]),
     "ce_swiglu": (_i, [_p, _p, _i, _i, _i, _p]),
     "ce_reluglu": (_i, [_p, _p, _i, _i, _i, _p]),

@@ -242,6 +242,7 @@ struct QkRopeArgs {
     int T, nh, nkv, d, rd, page_size, max_pages, num_pages, max_pos, write_kv;
     float eps;
     int pairing;             // partners of a rotation: 0 = (i, i + rd/2) ("rotate-half"), 1 = (2i, 2i + 1) (interleaved)
+    int weights_ready;       // no kernel in front writes q_weight and k_weight
 };
 
 template <typename T>
@@ -340,8 +341,8 @@ __device__ __forceinline__ void rope_store(T* p, const float (&v)[E]) {
 // the attention's merge in one trip 10,330 -> 10,040 (one request), 11,440 -> 11,152 (eight).
 template <typename T, int E, int L>
 __global__ void __launch_bounds__(128) qk_rope_kvwrite_warp_kernel(QkRopeArgs a, int hpw) {
-    // positions, slots, block tables, cosines, sines and norm weights are inputs of the step or constants:
-    // they are looked up while the kernel before this one (the QKV product) still runs; only its output waits
+    // positions, slots, block tables, cosines and sines are inputs of the step or constants: they are looked up while the kernel
+    // before this one (the QKV product) still runs.  Its output waits for it, and so do norm weights that a kernel may write.
     ce_pdl_launch_dependents();
     constexpr int AT_ONCE = 32 / L, SUMS = 32 / L, TERMS = E / SUMS;
     constexpr int W = E * sizeof(T) % 16 ? 8 / sizeof(T) : 16 / sizeof(T);
@@ -390,8 +391,9 @@ __global__ void __launch_bounds__(128) qk_rope_kvwrite_warp_kernel(QkRopeArgs a,
         held = w;
     };
     auto weights_of = [&](int hh) { return hh < a.nh ? a.q_weight : hh < a.nh + a.nkv ? a.k_weight : nullptr; };
-    hold(weights_of(hh0 + sub));
+    if (a.weights_ready) hold(weights_of(hh0 + sub));
     ce_pdl_wait();
+    hold(weights_of(hh0 + sub));
     constexpr int U = 2;                   // heads of a lane in flight together
     for (int hb = hh0; hb < hh1; hb += U * AT_ONCE) {
         float x1[U][E], x2[U][E];
@@ -478,7 +480,7 @@ extern "C" int ce_qk_rope_kvwrite(void* qkv, void* k_pool, void* v_pool, int dty
                                   const int* positions, const int* seq_of_token, const int* seq_slot,
                                   const int* block_table, int* status, int T, int nh, int nkv, int d, int rd,
                                   int page_size, int max_pages, int num_pages, int max_pos, int write_kv, float eps,
-                                  int pairing, cudaStream_t stream) {
+                                  int pairing, int weights_ready, cudaStream_t stream) {
     if (T == 0) return CE_OK;
     if (d <= 0 || d > 1024) return ce_fail(CE_ERR_SIZE, "ce_qk_rope_kvwrite: head_dim %d not in 1..1024", d);
     if (rd < 0 || rd > d || (rd & 1)) return ce_fail(CE_ERR_SIZE, "ce_qk_rope_kvwrite: rotary_dim %d must be even and <= head_dim %d", rd, d);
@@ -487,7 +489,8 @@ extern "C" int ce_qk_rope_kvwrite(void* qkv, void* k_pool, void* v_pool, int dty
     if (write_kv && (!k_pool || !v_pool || !seq_of_token || !seq_slot || !block_table))
         return ce_fail(CE_ERR_ARG, "ce_qk_rope_kvwrite: cache pointers missing");
     QkRopeArgs a{qkv, k_pool, v_pool, q_weight, k_weight, cos_table, sin_table, positions, seq_of_token, seq_slot,
-                 block_table, status, T, nh, nkv, d, rd, page_size, max_pages, num_pages, max_pos, write_kv, eps, pairing};
+                 block_table, status, T, nh, nkv, d, rd, page_size, max_pages, num_pages, max_pos, write_kv, eps, pairing,
+                 weights_ready};
     int threads = (d + 31) / 32 * 32;
     dim3 grid(T, nh + 2 * nkv);
     size_t smem = (d + 32) * sizeof(float);

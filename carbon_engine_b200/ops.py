@@ -239,9 +239,11 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, eps: float
 
 def qk_rope_kvwrite(qkv, k_pool, v_pool, q_weight, k_weight, cos, sin, positions, seq_of_token, seq_slot,
                     block_table, status, nh: int, nkv: int, d: int, rotary_dim: int, page_size: int,
-                    eps: float, write_kv: bool = True, pairing: str = "half") -> None:
+                    eps: float, write_kv: bool = True, pairing: str = "half", weights_ready: bool = False) -> None:
     """Per-head q/k RMSNorm, rotation, and the write of K and V into the pages.  ``pairing``: which elements
-    of a head turn together, "half" (i with i + rotary_dim/2) or "interleaved" (2i with 2i + 1)."""
+    of a head turn together, "half" (i with i + rotary_dim/2) or "interleaved" (2i with 2i + 1).  ``cos``, ``sin``, ``positions``
+    and the tables of slots and pages may be read while the kernels in front still run, so none of those may write them;
+    with ``weights_ready`` the norm weights too.  All other operands are read after them."""
     _need(qkv, "qkv")
     if pairing not in ROPE_PAIRINGS:
         raise KernelError(f"qk_rope_kvwrite: unknown pairing '{pairing}' (half, interleaved)")
@@ -264,7 +266,7 @@ def qk_rope_kvwrite(qkv, k_pool, v_pool, q_weight, k_weight, cos, sin, positions
         _ptr(qkv), _ptr(k_pool), _ptr(v_pool), dtype_code(qkv.dtype), _ptr(q_weight), _ptr(k_weight), _ptr(cos),
         _ptr(sin), _ptr(positions), _ptr(seq_of_token), _ptr(seq_slot), _ptr(block_table), _ptr(status),
         T, nh, nkv, d, rotary_dim, page_size, max_pages, num_pages, max_pos, 1 if write_kv else 0, float(eps),
-        ROPE_PAIRINGS[pairing], _stream()))
+        ROPE_PAIRINGS[pairing], int(weights_ready), _stream()))
 
 
 def add_residual(x: torch.Tensor, delta: torch.Tensor) -> None:

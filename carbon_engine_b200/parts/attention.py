@@ -135,7 +135,7 @@ class PagedAttention(Mixer):
                             ctx.positions, ctx.seq_of_token, ctx.seq_slot, table, ctx.status, nh, nkv, d,
                             pos.rotary_dim if cos is not None else 0, cache.page_size,
                             self.qk_norm_eps if self.qk_norm_eps is not None else 0.0, write_kv=cache.writes,
-                            pairing=pos.pairing if pos is not None else "half")
+                            pairing=pos.pairing if pos is not None else "half", weights_ready=True)
         out = ctx.buffer((T, nh * d))
         self.attend(ctx, qkv, out, cache, table)
         self.o.forward(out, x, ACCUM if accumulate else STORE_F32)

@@ -53,3 +53,34 @@ def test_the_norm_keeps_the_order_of_its_sums(dtype, nh, nkv, d, T):
     assert torch.equal(qkv.view(T, nh + 2 * nkv, d)[:, :nh], rms_norm(heads[:, :nh], qw).to(dtype))
     assert torch.equal(pool_rows(kp, table, positions, 16), rms_norm(heads[:, nh:nh + nkv], kw).to(dtype))
     assert torch.equal(pool_rows(vp, table, positions, 16), heads[:, nh + nkv:])
+
+
+@pytest.mark.parametrize("d", [64, 128, 192, 256])
+def test_norm_weights_that_the_kernel_in_front_makes(d):
+    """With dependent launches on: the product in front takes some 100 us, the rotation must not read its weights before it ends."""
+    from carbon_engine_b200 import ops
+    torch.manual_seed(d)
+    nh, nkv, T = 4, 2, 3
+    a, b = torch.randn(1024, 4096, device=dev()), torch.randn(512, 4096, device=dev())
+    made = torch.empty(1024, 512, device=dev())
+    table, kp, vp = paged_layout([T], 16, nkv, d, torch.float32)
+    source = torch.randn(T, (nh + 2 * nkv) * d, device=dev())
+    positions, sot, slots = step_meta([(0, T)])
+    st = status()
+
+    def rotate(qkv):
+        ops.qk_rope_kvwrite(qkv, kp, vp, made[1023, :d], made[1023, d:2 * d], None, None, positions, sot, slots, table, st, nh, nkv, d, 0, 16, EPS)
+
+    ops.set_dependent_launches(True)
+    ops.gemm_plain(a, b, made, ops.GEMM_STORE)
+    torch.cuda.synchronize()
+    want = source.clone()
+    rotate(want)
+    want_k = pool_rows(kp, table, positions, 16).clone()
+    for _ in range(5):
+        made.zero_()
+        got = source.clone()
+        torch.cuda.synchronize()
+        ops.gemm_plain(a, b, made, ops.GEMM_STORE)
+        rotate(got)                                                # (nothing between the two launches)
+        assert torch.equal(got, want) and torch.equal(pool_rows(kp, table, positions, 16), want_k)
