@@ -328,10 +328,41 @@ __device__ __forceinline__ void rope_store(T* p, const float (&v)[E]) {
     }
 }
 
+// The sum over L lanes with S sums each, as over L * S lanes with one (lane S * l + g: sum g of lane l) that add by halves, the lanes
+// furthest apart first.  A lane keeps half of its sums at each step, the other half is its partner's, until one is left (128 elements a
+// head: 6 shuffles, 12 with all sums kept); additions commute, so both partners' results are the same bits.
+template <int L, int S>
+__device__ __forceinline__ void rope_sum(float (&ss)[S], int lane) {
+    int n = S;
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) {
+        if (n > 1) {
+            n >>= 1;
+            const bool upper = lane & o;
+#pragma unroll
+            for (int g = 0; g < S / 2; ++g)
+                if (g < n) ss[g] = (upper ? ss[g + n] : ss[g]) + __shfl_xor_sync(0xffffffffu, upper ? ss[g] : ss[g + n], o);
+        } else {
+            ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], o);
+        }
+    }
+    // the sums that other lanes kept
+#pragma unroll
+    for (int o = L / 2, m = S; m > n; o >>= 1, m >>= 1)
+#pragma unroll
+        for (int g = 0; g < S; ++g)
+            if (g < n) ss[g] += __shfl_xor_sync(0xffffffffu, ss[g], o);
+#pragma unroll
+    for (int o = S / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int g = 0; g < o; ++g)
+            if (o < n) ss[g] += ss[g + o];
+}
+
 // Head sizes that are multiples of 64 (up to 256) with a full rotation.  A head belongs to L neighbouring lanes: a lane holds E
-// consecutive elements of the head's first half and the E elements d/2 further on, their partners in the rotation (E = 8, so accesses
-// of 16 bytes; heads of 192 take E = 12, which bfloat16 reads 8 bytes at a time), a warp takes 32 / L heads at a time, and nothing is
-// exchanged between lanes but the sum of squares.  The token's position, page, cosines and sines are looked up once per warp; a warp
+// consecutive elements of the head's first half and the E elements d/2 further on, their partners in the rotation, and moves W at a
+// time, 16 bytes where the operands start on them (the launcher says which E, L and W); a warp takes 32 / L heads at a time, and nothing
+// is exchanged between lanes but the sum of squares.  The token's position, page, cosines and sines are looked up once per warp; a warp
 // takes `hpw` consecutive heads of one token, as few as it takes at a time where tokens are few (decoding: as large a grid as can be),
 // a quarter of them all in portions of prompts.  A head's arithmetic does not depend on hpw.
 // The sum of squares is that of a warp of 32 lanes with d/64 elements of each half: such a lane's terms in order, first half then
@@ -339,13 +370,13 @@ __device__ __forceinline__ void rope_store(T* p, const float (&v)[E]) {
 // What bounds a long portion is the memory (2,048 tokens of 32 + 2 x 8 heads of 128: 50 MB in and out); with accesses of 4 bytes a lane it
 // was the instructions.  Measured: a prompt of 203 tokens, 12 layers of 8b sizes, 2,306 -> 2,243 us a pass; eight decode steps with this and
 // the attention's merge in one trip 10,330 -> 10,040 (one request), 11,440 -> 11,152 (eight).
-template <typename T, int E, int L>
+template <typename T, int E, int L, int W>
 __global__ void __launch_bounds__(128) qk_rope_kvwrite_warp_kernel(QkRopeArgs a, int hpw) {
     // positions, slots, block tables, cosines and sines are inputs of the step or constants: they are looked up while the kernel
     // before this one (the QKV product) still runs.  Its output waits for it, and so do norm weights that a kernel may write.
     ce_pdl_launch_dependents();
     constexpr int AT_ONCE = 32 / L, SUMS = 32 / L, TERMS = E / SUMS;
-    constexpr int W = E * sizeof(T) % 16 ? 8 / sizeof(T) : 16 / sizeof(T);
+    constexpr int WF = L == 32 ? W : E % 4 ? 2 : 4;              // of the float32 operands
     const int lane = threadIdx.x & 31, sub = lane / L, heads_per_token = a.nh + 2 * a.nkv;
     const int groups = (heads_per_token + hpw - 1) / hpw;
     const long long wg = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -367,8 +398,8 @@ __global__ void __launch_bounds__(128) qk_rope_kvwrite_warp_kernel(QkRopeArgs a,
 #pragma unroll
     for (int i = 0; i < E; ++i) { cs[i] = 1.f; sn[i] = 0.f; }
     if (rotate && hh0 < a.nh + a.nkv) {
-        rope_load<4>(a.cos_table + (size_t)pos * half + e0, cs);
-        rope_load<4>(a.sin_table + (size_t)pos * half + e0, sn);
+        rope_load<WF>(a.cos_table + (size_t)pos * half + e0, cs);
+        rope_load<WF>(a.sin_table + (size_t)pos * half + e0, sn);
     }
     size_t page_row = 0;
     if (hh1 > a.nh) {                      // a K or V head in this group: where the token's row lies in the pools
@@ -386,15 +417,15 @@ __global__ void __launch_bounds__(128) qk_rope_kvwrite_warp_kernel(QkRopeArgs a,
     const float* held = nullptr;           // the norm weights in w1 and w2
     auto hold = [&](const float* w) {
         if (!w || w == held) return;
-        rope_load<4>(w + e0, w1);
-        rope_load<4>(w + half + e0, w2);
+        rope_load<WF>(w + e0, w1);
+        rope_load<WF>(w + half + e0, w2);
         held = w;
     };
     auto weights_of = [&](int hh) { return hh < a.nh ? a.q_weight : hh < a.nh + a.nkv ? a.k_weight : nullptr; };
-    if (a.weights_ready) hold(weights_of(hh0 + sub));
-    ce_pdl_wait();
+    if (!a.weights_ready) ce_pdl_wait();
     hold(weights_of(hh0 + sub));
-    constexpr int U = 2;                   // heads of a lane in flight together
+    ce_pdl_wait();
+    constexpr int U = E > 4 ? 2 : 4;       // heads of a lane in flight together
     for (int hb = hh0; hb < hh1; hb += U * AT_ONCE) {
         float x1[U][E], x2[U][E];
 #pragma unroll
@@ -424,14 +455,7 @@ __global__ void __launch_bounds__(128) qk_rope_kvwrite_warp_kernel(QkRopeArgs a,
 #pragma unroll
                 for (int i = g * TERMS; i < (g + 1) * TERMS; ++i) ss[g] = fmaf(x2[u][i], x2[u][i], ss[g]);
             }
-#pragma unroll
-            for (int o = L / 2; o > 0; o >>= 1)
-#pragma unroll
-                for (int g = 0; g < SUMS; ++g) ss[g] += __shfl_xor_sync(0xffffffffu, ss[g], o);
-#pragma unroll
-            for (int o = SUMS / 2; o > 0; o >>= 1)
-#pragma unroll
-                for (int g = 0; g < o; ++g) ss[g] += ss[g + o];
+            rope_sum<L>(ss, lane);
             if (hh >= hh1) continue;
             T* dst = kv < 0 ? row + (size_t)hh * d : (T*)(v < 0 ? a.k_pool : a.v_pool) + (page_row + (size_t)(v < 0 ? kv : v) * a.page_size) * d;
             if (w) {
@@ -453,25 +477,54 @@ __global__ void __launch_bounds__(128) qk_rope_kvwrite_warp_kernel(QkRopeArgs a,
     }
 }
 
+// A head's lanes and accesses, and the elements that an operand must start on (0: not a head size of this kernel).  Operands on 16 bytes:
+// 4 float32 or 8 bfloat16 elements an access, and in steps of a few tokens, where latency is all, twice the lanes for a bfloat16 head
+// of 128 or 256 (one token of 32 + 2 x 8 heads of 128: 1.42 -> 1.35 us; 203 tokens 2.28 -> 2.6); heads of 192, whose lanes must hold whole
+// threes, 2.  Other operands: d / 64 elements an access (1 for heads of 192), 32 lanes (2,048 tokens: 14.2 us against 11.6; a block a
+// head took 102).
+struct RopeForm {
+    void (*kernel)(QkRopeArgs, int);
+    int lanes, start;
+};
+template <typename T>
+static RopeForm rope_form(int d, bool narrow, bool few) {
+    const bool four = sizeof(T) == 4;
+    switch (d) {
+        case 64:
+            if (narrow) return {qk_rope_kvwrite_warp_kernel<T, 1, 32, 1>, 32, 1};
+            if (four) return {qk_rope_kvwrite_warp_kernel<T, 4, 8, 4>, 8, 4};
+            return {qk_rope_kvwrite_warp_kernel<T, 8, 4, 8>, 4, 8};
+        case 128:
+            if (narrow) return {qk_rope_kvwrite_warp_kernel<T, 2, 32, 2>, 32, 2};
+            if (four || few) return {qk_rope_kvwrite_warp_kernel<T, 4, 16, 4>, 16, 4};
+            return {qk_rope_kvwrite_warp_kernel<T, 8, 8, 8>, 8, 8};
+        case 192:
+            if (narrow) return {qk_rope_kvwrite_warp_kernel<T, 3, 32, 1>, 32, 1};
+            return {qk_rope_kvwrite_warp_kernel<T, 6, 16, 2>, 16, 2};
+        case 256:
+            if (narrow || four || few) return {qk_rope_kvwrite_warp_kernel<T, 4, 32, 4>, 32, 4};
+            return {qk_rope_kvwrite_warp_kernel<T, 8, 16, 8>, 16, 8};
+    }
+    return {nullptr, 32, 1};
+}
+
 template <typename T>
 static bool launch_rope_warp(const QkRopeArgs& a, cudaStream_t stream) {
-    const int heads_per_token = a.nh + 2 * a.nkv;
-    if (a.d % 64 || a.d > 256 || (a.cos_table && (a.rd != a.d || a.pairing != 0))) return false;
-    if (((uintptr_t)a.qkv | (uintptr_t)a.k_pool | (uintptr_t)a.v_pool | (uintptr_t)a.q_weight | (uintptr_t)a.k_weight |
-         (uintptr_t)a.cos_table | (uintptr_t)a.sin_table) & 15) return false;                 // (accesses of 16 bytes)
-    const int lanes = a.d == 64 ? 4 : a.d == 256 ? 16 : 8, at_once = 32 / lanes;
-    // few tokens: as many warps as there are; many: four warps share a token's heads
-    const int hpw = a.T >= 256 ? ((heads_per_token + 3) / 4 + at_once - 1) / at_once * at_once : at_once;
+    if (a.cos_table && (a.rd != a.d || a.pairing != 0)) return false;
+    const uintptr_t rows = (uintptr_t)a.qkv | (uintptr_t)a.k_pool | (uintptr_t)a.v_pool;
+    const uintptr_t floats = (uintptr_t)a.q_weight | (uintptr_t)a.k_weight | (uintptr_t)a.cos_table | (uintptr_t)a.sin_table;
+    const RopeForm form = rope_form<T>(a.d, (rows | floats) % 16, a.T < 64);
+    if (!form.kernel || rows % 16 % (form.start * sizeof(T)) || floats % 16 % (form.start * sizeof(float))) return false;
+    const int heads_per_token = a.nh + 2 * a.nkv, at_once = 32 / form.lanes;
+    // few tokens: as many warps as there are, while the chip takes them at once; many: four warps share a token's heads
+    int hpw = at_once;
+    if (a.T >= 256) hpw = ((heads_per_token + 3) / 4 + at_once - 1) / at_once * at_once;
+    else
+        while (hpw < 4 && (long long)a.T * ((heads_per_token + hpw - 1) / hpw) > 32 * 148) hpw *= 2;
     const long long warps = (long long)a.T * ((heads_per_token + hpw - 1) / hpw);
     if ((warps + 3) / 4 > 2147483647LL) return false;
-    const unsigned blocks = (unsigned)((warps + 3) / 4);
     ce_note("qk_rope_kvwrite_warp_kernel");
-    switch (a.d) {
-        case 64: ce_launch(qk_rope_kvwrite_warp_kernel<T, 8, 4>, blocks, 128, 0, stream, a, hpw); break;
-        case 128: ce_launch(qk_rope_kvwrite_warp_kernel<T, 8, 8>, blocks, 128, 0, stream, a, hpw); break;
-        case 192: ce_launch(qk_rope_kvwrite_warp_kernel<T, 12, 8>, blocks, 128, 0, stream, a, hpw); break;
-        default: ce_launch(qk_rope_kvwrite_warp_kernel<T, 8, 16>, blocks, 128, 0, stream, a, hpw); break;
-    }
+    ce_launch(form.kernel, (unsigned)((warps + 3) / 4), 128, 0, stream, a, hpw);
     return true;
 }
 

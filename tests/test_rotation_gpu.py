@@ -84,3 +84,44 @@ def test_norm_weights_that_the_kernel_in_front_makes(d):
         ops.gemm_plain(a, b, made, ops.GEMM_STORE)
         rotate(got)                                                # (nothing between the two launches)
         assert torch.equal(got, want) and torch.equal(pool_rows(kp, table, positions, 16), want_k)
+
+
+def shifted(t, by):
+    """The same values from `by` bytes behind a 16-byte boundary on."""
+    room = torch.empty(t.numel() + 16, dtype=t.dtype, device=t.device)
+    room = room[by // t.element_size():][:t.numel()].view(t.shape)
+    room.copy_(t)
+    assert room.data_ptr() % 16 == by % 16
+    return room
+
+
+# the smallest accesses: d / 64 elements, single elements of heads of 192 (bfloat16: 2, 4, 2, 8 bytes; float32: 4, 8, 4, 16)
+@pytest.mark.parametrize("nh,nkv,d,by", [(4, 2, 64, {2: 2, 4: 4}), (5, 1, 128, {2: 4, 4: 8}), (3, 2, 192, {2: 2, 4: 4}), (4, 2, 256, {2: 8})])
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("which", ["qkv", "pools", "floats", "all"])
+@pytest.mark.parametrize("T", [5, 260])
+def test_operands_between_16_byte_boundaries(dtype, nh, nkv, d, by, which, T):
+    """The same kernel and the same bits as with operands that start on 16 bytes."""
+    from carbon_engine_b200 import ops
+    size = torch.empty(0, dtype=dtype).element_size()
+    if size not in by:
+        pytest.skip("its accesses are of 16 bytes")
+    torch.manual_seed(d + T)
+    table, kp, vp = paged_layout([T], 16, nkv, d, dtype)
+    qkv = torch.randn(T, (nh + 2 * nkv) * d, device=dev()).to(dtype)
+    qw, kw = 1 + 0.2 * torch.randn(d, device=dev()), 1 + 0.2 * torch.randn(d, device=dev())
+    angles = torch.rand(T, d // 2, device=dev())
+    positions, sot, slots = step_meta([(0, T)])
+    floats_by = {64: 4, 128: 8, 192: 4, 256: 0}[d]
+
+    def rotate(move):
+        row = lambda t, name: shifted(t, by[size] if move in (name, "all") else 0)
+        vec = lambda t: shifted(t, floats_by if move in ("floats", "all") else 0)
+        x, k, v = row(qkv, "qkv"), row(kp, "pools"), row(vp, "pools")
+        before, st = ops.kernel_counts().get(NAME, 0), status()
+        ops.qk_rope_kvwrite(x, k, v, vec(qw), vec(kw), vec(angles.cos()), vec(angles.sin()), positions, sot, slots, table, st, nh, nkv, d, d, 16, EPS)
+        assert ops.kernel_counts().get(NAME, 0) == before + 1 and st.item() == 0
+        return x, pool_rows(k, table, positions, 16), pool_rows(v, table, positions, 16)
+
+    for got, want in zip(rotate(which), rotate(None)):
+        assert torch.equal(got, want)
