@@ -22,6 +22,12 @@ _SUBMIT_ERRORS = {
 }
 
 
+def _c_array(values: np.ndarray, kind):
+    """The array's values for a native call.  (numpy, which refuses what does not fit, has converted them: a ctypes array made from
+    Python's numbers would cut them to size.  A copy of a few numbers is cheaper than numpy's ctypes pointer.)"""
+    return (kind * values.size).from_buffer_copy(values)
+
+
 class SubmitError(ValueError):
     pass
 
@@ -79,9 +85,9 @@ class Scheduler:
     def plan_for(self, request_ids: Sequence[int]) -> List[PlanEntry]:
         """The step that is already on the device for ``request_ids`` (one token each, fed there from the last
         step's picks): its entries for those of them that still run.  Nothing is admitted."""
-        n_ids = len(request_ids)
+        ids = np.ascontiguousarray(request_ids, dtype=np.int64)
         n_tok = ctypes.c_int(0)
-        n = self._lib.sched_plan_for(self._h, (ctypes.c_int64 * n_ids)(*request_ids), n_ids, self._p_entries, len(self._entries) // 5,
+        n = self._lib.sched_plan_for(self._h, _c_array(ids, ctypes.c_int64), len(ids), self._p_entries, len(self._entries) // 5,
                                      self._p_tokens, len(self._tokens), ctypes.byref(n_tok))
         return self._read_plan(n, n_tok.value)
 
@@ -109,8 +115,8 @@ class Scheduler:
         return self._lib.sched_running(self._h)
 
     def commit(self, sampled: Sequence[int]) -> None:
-        n = len(sampled)
-        if self._lib.sched_commit(self._h, (ctypes.c_int32 * n)(*sampled), n) != 0:
+        s = np.ascontiguousarray(sampled, dtype=np.int32)
+        if self._lib.sched_commit(self._h, _c_array(s, ctypes.c_int32), len(s)) != 0:
             raise RuntimeError("commit: the number of sampled tokens does not match the plan")
 
     def fail_step(self) -> None:

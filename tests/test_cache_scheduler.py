@@ -168,6 +168,24 @@ def test_prompts_are_cut_under_the_budget_and_decoders_go_first():
     assert cm.free_pages() == 32 and cm.free_slots() == 4
 
 
+def test_numbers_beyond_the_native_types_are_refused():
+    """2**32 + 5 is not token 5, 2**64 + 1 is not request 1: the step stays as it was."""
+    cm, s = make()
+    s.submit(1, [1, 2], max_tokens=4)
+    s.plan()
+    for wide in (2 ** 32 + 5, 2 ** 31, -2 ** 40):
+        with pytest.raises(OverflowError):
+            s.commit([wide])
+    s.commit(np.array([5]))
+    for wide in (2 ** 64 + 1, 2 ** 63):
+        with pytest.raises(OverflowError):
+            s.plan_for([wide])
+    assert s.tokens_of(1) == [1, 2, 5]
+    assert [(e.request_id, e.tokens) for e in s.plan_for([1])] == [(1, [5])]
+    s.commit([6])
+    assert s.tokens_of(1) == [1, 2, 5, 6] and s.plan_for([]) == []
+
+
 def test_a_decoding_request_is_never_starved_by_prompts():
     cm, s = make(pages=64, budget=6, max_seq_len=128)
     s.submit(1, [1, 2], max_tokens=20)
