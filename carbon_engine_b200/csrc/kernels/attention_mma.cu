@@ -71,6 +71,7 @@ struct MmaAttnArgs {
     int* status;
     int nh, nkv, d, q_stride, page_size, max_pages, num_pages, window, max_splits, split, fused_merge;
     int longest_first;          // TMA decode kernel: clusters take the sequences by their lengths, the longest first
+    int overlap;                // TMA decode kernel: kernels behind may start before this one ends
     int cluster_merge;          // TMA decode kernel: the splits of a sequence form a cluster and merge through shared memory
     float scale_log2;           // scale * log2(e)
     const float* sinks;         // [nh] or null: exp(sinks[h]) joins head h's denominator, with no key and no value
@@ -561,7 +562,7 @@ __global__ void __launch_bounds__(AMT_THREADS) attention_decode_tma_kernel(const
     // the block looks up its pages and starts the copies of all tiles except the one that holds the
     // newest key while the kernels before it still run; only that tile, the query and everything the
     // block writes wait for them.
-    ce_pdl_launch_dependents();
+    if (a.overlap) ce_pdl_launch_dependents();
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[ST], empty_bar[ST];
     int split = blockIdx.x % a.max_splits, b = blockIdx.x / a.max_splits, kvh = blockIdx.y, hg = blockIdx.z;
@@ -570,7 +571,7 @@ __global__ void __launch_bounds__(AMT_THREADS) attention_decode_tma_kernel(const
         // Clusters start in the order of their numbers, as room becomes free: sequences with the most keys first (all KV heads of one,
         // then the next), so that the last to start are the shortest.  The order is taken from the positions, which are there anyway.
         // (21 sequences of 450 to 9,000 keys, 8 KV heads, a pass of four steps of 12 layers: 10.42 ms as the batch has them, cut at shares of
-        // the longest context; 10.46 with the order alone, 9.51 with a sequence's own shares alone, 8.33 with both.)
+        // the longest context; 10.46 with the order alone, 9.51 with a sequence's own shares alone, 8.33 with both, 8.56 since such a grid stands alone.)
         __shared__ __align__(16) int s_pos[AMT_MAX_SORTED];
         __shared__ int s_b;
         const int n = gridDim.x / a.max_splits, at = blockIdx.y * n + b, rank = at / a.nkv;
@@ -984,6 +985,38 @@ template <typename F> static int set_smem(F kernel, size_t bytes, const char* wh
     return CE_OK;
 }
 
+// One launch of the TMA decode kernel.  Clusters stand alone where there are more of them than the chip holds (ce_clusters_at_once):
+// 21 sequences x 8 KV heads of up to 9,000 keys are 168 clusters of 3 where 93 have room (a pass of four steps of 12 layers 8.41 -> 8.56 ms).
+template <int DM, int ST, bool BIAS>
+static int launch_decode_tma(const CUtensorMap& mk, const CUtensorMap& mv, MmaAttnArgs a, int box_rows, dim3 grid, size_t smem, cudaStream_t stream) {
+    int rc = set_smem(attention_decode_tma_kernel<DM, ST, BIAS>, smem, "ce_attention_decode_bf16");
+    if (rc) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(AMT_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
+    a.overlap = 1;
+    if (a.cluster_merge) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = a.max_splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.numAttrs = 1;
+        static CeRoom room[2][9];                       // (heads of 192 and of 256 share an instantiation, not their shared memory)
+        if (a.max_splits > 1)
+            a.overlap = (long long)grid.x / a.max_splits * grid.y * grid.z <=
+                        ce_clusters_at_once(room[a.d == DM][a.max_splits], attention_decode_tma_kernel<DM, ST, BIAS>, cfg);
+    }
+    if (a.overlap && ce_pdl_enabled()) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, attention_decode_tma_kernel<DM, ST, BIAS>, mk, mv, a, box_rows);
+    if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_attention_decode_bf16: %s", cudaGetErrorString(e));
+    return ce_check_launch("ce_attention_decode_bf16");
+}
+
 // Scratch floats the decode kernel needs for n_seqs sequences.
 extern "C" long long ce_attention_decode_scratch(int n_seqs, int nh, int d, int max_splits) {
     return (long long)n_seqs * nh * max_splits * (d + 2);
@@ -1110,39 +1143,16 @@ extern "C" int ce_attention_decode_bf16_sink(const void* q, const void* k_pool, 
         tsmem += 1024;
         a.cluster_merge = use_cluster;
         a.longest_first = use_cluster && n_seqs > 1 && n_seqs <= AMT_MAX_SORTED;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = grid;
-        cfg.blockDim = dim3(AMT_THREADS);
-        cfg.dynamicSmemBytes = tsmem;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[2];
-        int n_attr = 0;
-        if (ce_pdl_enabled()) {
-            attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
-            ++n_attr;
-        }
-        if (a.cluster_merge) {
-            attr[n_attr].id = cudaLaunchAttributeClusterDimension;
-            attr[n_attr].val.clusterDim.x = max_splits; attr[n_attr].val.clusterDim.y = 1; attr[n_attr].val.clusterDim.z = 1;
-            ++n_attr;
-        }
-        cfg.attrs = attr;
-        cfg.numAttrs = n_attr;
-        cudaError_t le = cudaSuccess;
         ce_note(a.cluster_merge ? "attention_decode_tma_kernel (merge in the cluster)" : "attention_decode_tma_kernel");
-#define AMT_LAUNCH(DM, ST, BIAS)                                                                                       \
-        {                                                                                                              \
-            if ((rc = set_smem(attention_decode_tma_kernel<DM, ST, BIAS>, tsmem, "ce_attention_decode_bf16"))) return rc; \
-            le = cudaLaunchKernelEx(&cfg, attention_decode_tma_kernel<DM, ST, BIAS>, mk, mv, a, box_rows);              \
-        }
         // three stages for heads of up to 128 (deep3), two above
-#define AMT_CASE(DM, ST) if (slopes) AMT_LAUNCH(DM, ST, true) else AMT_LAUNCH(DM, ST, false)
-        if (d == 64) { AMT_CASE(64, 3) } else if (d == 128) { AMT_CASE(128, 3) } else { AMT_CASE(256, 2) }
+#define AMT_LAUNCH(DM, ST)                                                                              \
+        rc = slopes ? launch_decode_tma<DM, ST, true>(mk, mv, a, box_rows, grid, tsmem, stream)         \
+                    : launch_decode_tma<DM, ST, false>(mk, mv, a, box_rows, grid, tsmem, stream)
+        if (d == 64) AMT_LAUNCH(64, 3);
+        else if (d == 128) AMT_LAUNCH(128, 3);
+        else AMT_LAUNCH(256, 2);
 #undef AMT_LAUNCH
-#undef AMT_CASE
-        if (le != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_attention_decode_bf16: %s", cudaGetErrorString(le));
-        if ((rc = ce_check_launch("ce_attention_decode_bf16"))) return rc;
+        if (rc) return rc;
         g_decode_launches = a.cluster_merge ? 1 : 2;
         if (a.cluster_merge) return CE_OK;
         { ce_note("attention_merge_kernel"); ce_launch(attention_merge_kernel, dim3(n_seqs, nh), d >= 128 ? 128 : (d + 31) / 32 * 32, max_splits * sizeof(float), stream, a); }

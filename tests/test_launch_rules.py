@@ -27,7 +27,7 @@ def linked(tmp_path_factory):
         pytest.skip("no CUDA toolkit")
     cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
     headers = build._sources(build.KERNEL_DIR, (".cuh", ".h"))
-    names = ("errors", "tensor_map", "gemm_tc", "gemm_f32", "gemm_plain", "attention_f32")
+    names = ("errors", "tensor_map", "gemm_tc", "gemm_f32", "gemm_plain", "attention_f32", "attention_mma")
     objects = build._compile_all(nvcc, build.NVCC_FLAGS, [os.path.join(build.KERNEL_DIR, n + ".cu") for n in names], headers, build.build_dir(), "k")
     out = str(tmp_path_factory.mktemp("fake") / "libfake.so")
     cxx = os.environ.get("CXX") or shutil.which("g++") or shutil.which("c++")
@@ -69,6 +69,12 @@ class Chip:
         p = ctypes.c_void_p(ADDR)
         return self._launched(self.lib.ce_attention_f32(*[p] * 10, n_decode, n_tiles, heads, kv_heads, d, heads * d, 64, 100, 100, 0, longest,
                                                         ctypes.c_float(1), None))
+
+    def decode(self, n, longest, heads=32, kv_heads=8, d=128, page=64, slopes=None):
+        p = ctypes.c_void_p(ADDR)
+        return self._launched(self.lib.ce_attention_decode_bf16_sink(
+            *[p] * 6, 1 << 20, *[p] * 6, n, heads, kv_heads, d, (heads + 2 * kv_heads) * d, page, 200, 1000, 0, ctypes.c_float(1),
+            (longest + 127) // 128, None, ctypes.c_float(1), slopes, None))
 
 
 B200 = {2: 74, 3: 60, 4: 33, 5: 30, 6: 22, 7: 20, 8: 15}
@@ -137,6 +143,29 @@ def test_more_clusters_than_the_chip_holds_stand_alone(linked, room, overlaps):
     chip = Chip(linked, {8: room})
     for seen in (chip.gemm_f32(4, 2048, 2048), chip.attention_f32(4, 0)):
         assert seen.cluster[2] == seen.grid[2] == 8 and bool(seen.dependent) == overlaps
+
+
+# sequences, longest context, head size: 2 to 6 blocks a cluster; 8 KV heads
+@pytest.mark.parametrize("n,longest,d,blocks", [(21, 9000, 128, 3), (16, 2304, 128, 2), (8, 2304, 64, 4), (1, 2304, 192, 6), (1, 2304, 256, 6)])
+@pytest.mark.parametrize("spare", [0, -1])
+@pytest.mark.parametrize("slopes", [None, ctypes.c_void_p(ADDR)])
+def test_decode_attention_of_more_clusters_than_the_chip_holds_stands_alone(linked, n, longest, d, blocks, spare, slopes):
+    seen = Chip(linked, {blocks: 8 * n + spare}).decode(n, longest, d=d, slopes=slopes)
+    assert b"attention_decode_tma_kernel" in seen.kernel and seen.cluster[0] == blocks and seen.grid[0] == n * blocks
+    assert bool(seen.dependent) == (spare == 0)
+
+
+def test_decode_attention_of_one_block_a_sequence_overlaps(linked):
+    chip = Chip(linked, {1: 1})
+    seen = chip.decode(64, 2304)
+    assert seen.cluster[0] == 1 and seen.dependent and chip.lib.fake_occupancy_calls() == 0
+
+
+def test_heads_of_192_and_256_are_asked_for_apart(linked):
+    chip = Chip(linked, {6: 100})
+    for d in (192, 256, 192, 256):
+        chip.decode(1, 2304, d=d)
+    assert chip.lib.fake_occupancy_calls() == 2
 
 
 def test_without_room_for_a_cluster_the_float32_kernels_run_without(linked):
