@@ -111,6 +111,11 @@ def run() -> int:
     ops.argmax(logits, out)
     want = [int(logits[0].argmax()), 77, int(logits[2].argmax())]
     check("greedy pick (first maximum)", 0.0 if out.tolist() == want else 1.0, 0.0)
+    # the float32 product of a decode step
+    a, wm = torch.randn(4, 2048, device=dev), torch.randn(2048, 2048, device=dev) / 45
+    c = torch.empty(4, 2048, device=dev)
+    ops.gemm_plain(a, wm, c, ops.GEMM_STORE)
+    check("product of a few tokens f32", _rel(c, a.double() @ wm.double().T), 1e-5)
     # tensor-core kernels
     a = torch.randn(24, 512, device=dev).to(torch.bfloat16)
     wm = (torch.randn(300, 512, device=dev) / 20).to(torch.bfloat16)
@@ -146,7 +151,7 @@ def run() -> int:
     for name in sorted(launched):
         print(f"  {name}: {launched[name]}")
     for name in ("attention_decode_tma_kernel (merge in the cluster)", "attention_prefill_tc_kernel", "gemm_tc_pair_kernel",
-                 "gemm_tc_kernel (split-K, splits add together)", "gemm_f32_kernel", "attention_f32_kernel",
+                 "gemm_tc_kernel (split-K, splits add together)", "gemm_f32_kernel", "gemm_f32_stream_kernel", "attention_f32_kernel",
                  "attention_f32_kernel (stripes in a cluster)", "sample_kernel"):
         if launched.get(name, 0) == 0:
             failures.append(f"{name} was never launched")

@@ -83,6 +83,27 @@ def test_float32_product_reads_a_matrix_that_the_kernel_in_front_makes(M):
         assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("M", [3, 8])
+def test_float32_stream_product_reads_a_matrix_that_the_kernel_in_front_makes(M):
+    """The same at sizes of the kernel that streams weights for up to 8 tokens; the product in front takes some 350 us."""
+    from carbon_engine_b200 import ops
+    torch.manual_seed(5)
+    a, b, x = torch.randn(1024, 2304, device=dev()), torch.randn(2048, 2304, device=dev()), torch.randn(M, 2048, device=dev())
+    made = torch.zeros(1024, 2048, device=dev())
+    ops.set_dependent_launches(True)
+    ops.gemm_plain(a, b, made, ops.GEMM_STORE)
+    torch.cuda.synchronize()
+    want, got = product(x, made, ops.GEMM_STORE), torch.empty(M, 1024, device=dev())
+    for _ in range(5):
+        made.zero_()
+        torch.cuda.synchronize()
+        before = ops.kernel_counts().get("gemm_f32_stream_kernel", 0)
+        ops.gemm_plain(a, b, made, ops.GEMM_STORE)
+        ops.gemm_plain(x, made, got, ops.GEMM_STORE)               # (nothing between the two launches)
+        assert ops.kernel_counts().get("gemm_f32_stream_kernel", 0) == before + 1
+        assert torch.equal(got, want)
+
+
 def attention(seqs, q, kp, vp, table, nh, nkv, d, ps, window, stride):
     from carbon_engine_b200 import ops
     T = sum(n for _, n in seqs)

@@ -125,3 +125,39 @@ def test_operands_between_16_byte_boundaries(dtype, nh, nkv, d, by, which, T):
 
     for got, want in zip(rotate(which), rotate(None)):
         assert torch.equal(got, want)
+
+
+# more heads than a warp takes at once, not a multiple of them: a warp's heads change from query to key to value on the way
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("nh,nkv,d", [(70, 3, 64), (19, 3, 128), (19, 3, 192), (19, 3, 256)])
+def test_a_heads_bits_do_not_depend_on_the_steps_tokens(dtype, nh, nkv, d):
+    """Steps of fewer than 64, of fewer than 256 and of more tokens walk over a token's heads in different portions."""
+    from carbon_engine_b200 import ops
+    torch.manual_seed(d)
+    T, ps = 400, 16
+    table, kp, vp = paged_layout([T], ps, nkv, d, dtype)
+    qkv = torch.randn(T, (nh + 2 * nkv) * d, device=dev()).to(dtype)
+    qw, kw = 1 + 0.2 * torch.randn(d, device=dev()), 1 + 0.2 * torch.randn(d, device=dev())
+    angles = torch.rand(T, d // 2, device=dev()) * 6
+    cos, sin, st = angles.cos(), angles.sin(), status()
+
+    def steps(cuts):
+        k, v, rows, start = kp.clone(), vp.clone(), [], 0
+        for n in cuts:
+            positions, sot, slots = step_meta([(start, n)])
+            x = qkv[start:start + n].clone()
+            ops.qk_rope_kvwrite(x, k, v, qw, kw, cos, sin, positions, sot, slots, table, st, nh, nkv, d, d, ps, EPS)
+            rows.append(x[:, :nh * d])
+            start += n
+        assert start == T and st.item() == 0
+        return torch.cat(rows), k, v
+
+    whole = steps([400])
+    assert int((~torch.isnan(whole[1].float())).sum()) == T * nkv * d
+    for cuts in ([255, 63, 64, 1, 17], [256, 144]):
+        for got, want in zip(steps(cuts), whole):
+            assert torch.equal(torch.nan_to_num(got), torch.nan_to_num(want))
+    # a layer that reads another's cache: queries alone
+    x = qkv[:300].clone()
+    ops.qk_rope_kvwrite(x, None, None, qw, kw, cos, sin, step_meta([(0, 300)])[0], None, None, None, st, nh, nkv, d, d, ps, EPS, write_kv=False)
+    assert st.item() == 0 and torch.equal(x[:, :nh * d], whole[0][:300]) and torch.equal(x[:, nh * d:], qkv[:300, nh * d:])
