@@ -8,13 +8,19 @@
 // into a ring of its own (cp.async, no barrier of the block inside the loop), a lane holds whole rows, and the eight runs meet in
 // shared memory once.
 // Measured: four decode steps of four layers (width 2,048, 4 requests of 350 to 700 tokens) 1,592 us with the clusters -> 1,430.
+// One product (weight rows x K), us with the clusters -> here, weights from memory:
+//                   2,048 x 2,048    2,560 x 9,728    4,096 x 4,096    4,096 x 12,288    5,120 x 5,120    12,288 x 2,048 (gated)
+//     1 token        7.3 -> 6.1       33.3 -> 25.7     16.4 -> 12.7      42.9 -> 34.9      20.1 -> 19.5     22.5 -> 16.9
+//     8 tokens      10.2 -> 7.6       47.1 -> 41.0     22.5 -> 18.1      60.3 -> 49.4      27.9 (there)     28.4 -> 22.3
 #include "gemm_f32.cuh"
+#include <type_traits>
 
 namespace {
 
 constexpr int FS_RUNS = 8;                              // runs of K = warps of a block
 constexpr int FS_THREADS = 32 * FS_RUNS;
-constexpr int FS_BLOCKS = 148;                          // blocks the rows are dealt to
+constexpr size_t FS_ALONE = 116 * 1024;                  // more than half of an SM's shared memory
+constexpr size_t FS_MOST = 196 * 1024;                  // bytes of a block's rings
 
 struct FsArgs {
     const float* A;
@@ -34,8 +40,19 @@ __device__ __forceinline__ void fs_cp16(float* dst, const float* src, bool in) {
 template <int KS>
 __device__ __forceinline__ int fs_at(int r, int c) { return r * KS + ((KS == 32 ? c ^ (r & 7) : c ^ ((r >> 1) & 3)) << 2); }
 
-// RT: rows a lane holds; LT: groups of lanes with tokens of their own (2 where a block has at most 16 rows); TOK: tokens; KS: k of a stage.
-template <int RT, int LT, int TOK, int KS, bool GATED>
+// Stages of a warp's ring: up to eight, as many as 150 KB hold, four or three where those need more.  (14 rows and 4 tokens: eight stages,
+// 147 KB, 1,433 us a pass of four decode steps of four layers; four stages, 1,579.  2,560 x 9,728, where six fit: 25.7 us, with four 39.4,
+// with the clusters 33.4.)
+__host__ __device__ constexpr size_t fs_stage_bytes(int wrows, int tok, int ks) { return sizeof(float) * FS_RUNS * (wrows + tok) * ks; }
+__host__ __device__ constexpr int fs_stages(int wrows, int tok, int ks) {
+    const size_t stage = fs_stage_bytes(wrows, tok, ks);
+    const int n = (int)(150 * 1024 / stage);
+    return n > 8 ? 8 : n >= 4 ? n : 4 * stage <= FS_MOST ? 4 : 3;
+}
+
+// RT: rows a lane holds; LT: groups of lanes with tokens of their own, so that a warp holds 32 / LT x RT rows (of fewer, lanes
+// multiply padding: a block of FIRST rows does the work of 32 / LT x RT); TOK: tokens; KS: k of a stage.
+template <int RT, int LT, int FIRST, int TOK, int KS, bool GATED>
 __global__ void __launch_bounds__(FS_THREADS, 2) gemm_f32_stream_kernel(FsArgs a) {
     extern __shared__ __align__(128) float fs_smem[];
     constexpr int PIECES = KS / 4, LR = 32 / LT, TT = TOK / LT, STEP = 32 / PIECES;
@@ -81,35 +98,46 @@ __global__ void __launch_bounds__(FS_THREADS, 2) gemm_f32_stream_kernel(FsArgs a
     int row[RT];
 #pragma unroll
     for (int j = 0; j < RT; ++j) row[j] = min(lr + LR * j, wrows - 1);               // (lanes beyond the rows: any, not stored)
-    int slot = 0, next = a.stages - 1;
-    for (int s = 0; s < slabs; ++s) {
-        // this warp's copies alone: all but the newest stages - 2 groups have landed
-        if (a.stages == 8) asm volatile("cp.async.wait_group 6;" ::: "memory");
-        else if (a.stages == 4) asm volatile("cp.async.wait_group 2;" ::: "memory");
-        else asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncwarp();
-        if (s + a.stages - 1 < slabs) { load_w(s + a.stages - 1, next); load_x(s + a.stages - 1, next); }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        const float* wt = ring + slot * stage;
-        const float* xt = wt + wrows * KS;
+    auto walk = [&](auto depth) {
+        constexpr int ST = decltype(depth)::value;
+        int slot = 0, next = ST - 1;
+        for (int s = 0; s < slabs; ++s) {
+            // this warp's copies alone: all but the newest ST - 2 groups have landed
+            asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+            __syncwarp();
+            if (s + ST - 1 < slabs) { load_w(s + ST - 1, next); load_x(s + ST - 1, next); }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            const float* wt = ring + slot * stage;
+            const float* xt = wt + wrows * KS;
 #pragma unroll(RT * TT >= 8 ? 2 : 4)
-        for (int q = 0; q < PIECES; ++q) {
-            float4 w[RT];
+            for (int q = 0; q < PIECES; ++q) {
+                float4 w[RT];
 #pragma unroll
-            for (int j = 0; j < RT; ++j) w[j] = *reinterpret_cast<const float4*>(wt + fs_at<KS>(row[j], q));
+                for (int j = 0; j < RT; ++j) w[j] = *reinterpret_cast<const float4*>(wt + fs_at<KS>(row[j], q));
 #pragma unroll
-            for (int m = 0; m < TT; ++m) {
-                const float4 x = *reinterpret_cast<const float4*>(xt + fs_at<KS>(lt * TT + m, q));
+                for (int m = 0; m < TT; ++m) {
+                    const float4 x = *reinterpret_cast<const float4*>(xt + fs_at<KS>(lt * TT + m, q));
 #pragma unroll
-                for (int j = 0; j < RT; ++j) {
-                    acc[j][m] = __ffma2_rn(make_float2(x.x, x.y), make_float2(w[j].x, w[j].y), acc[j][m]);
-                    acc[j][m] = __ffma2_rn(make_float2(x.z, x.w), make_float2(w[j].z, w[j].w), acc[j][m]);
+                    for (int j = 0; j < RT; ++j) {
+                        acc[j][m] = __ffma2_rn(make_float2(x.x, x.y), make_float2(w[j].x, w[j].y), acc[j][m]);
+                        acc[j][m] = __ffma2_rn(make_float2(x.z, x.w), make_float2(w[j].z, w[j].w), acc[j][m]);
+                    }
                 }
             }
+            next = slot;
+            if (++slot == ST) slot = 0;
+            __syncwarp();                               // the slot just read takes the next copies
         }
-        next = slot;
-        if (++slot == a.stages) slot = 0;
-        __syncwarp();                                   // the slot just read takes the next copies
+    };
+    // (the number of groups to wait for is part of the instruction: a loop for each depth that these rows can have)
+    constexpr int LEAST = fs_stages(32 / LT * RT, TOK, KS), MOST = fs_stages(FIRST, TOK, KS);
+    switch (a.stages) {
+        case 8: if constexpr (LEAST <= 8 && MOST >= 8) walk(std::integral_constant<int, 8>{}); break;
+        case 7: if constexpr (LEAST <= 7 && MOST >= 7) walk(std::integral_constant<int, 7>{}); break;
+        case 6: if constexpr (LEAST <= 6 && MOST >= 6) walk(std::integral_constant<int, 6>{}); break;
+        case 5: if constexpr (LEAST <= 5 && MOST >= 5) walk(std::integral_constant<int, 5>{}); break;
+        case 4: if constexpr (LEAST <= 4 && MOST >= 4) walk(std::integral_constant<int, 4>{}); break;
+        case 3: if constexpr (LEAST <= 3 && MOST >= 3) walk(std::integral_constant<int, 3>{}); break;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
@@ -150,49 +178,55 @@ __global__ void __launch_bounds__(FS_THREADS, 2) gemm_f32_stream_kernel(FsArgs a
     }
 }
 
-template <int RT, int LT, int TOK, int KS, bool GATED>
+template <int RT, int LT, int FIRST, int TOK, int KS, bool GATED>
 int fs_launch(const FsArgs& a, size_t smem, cudaStream_t stream) {
     static std::atomic<unsigned long long> allowed{0};
-    cudaError_t e = ce_allow_smem(allowed, gemm_f32_stream_kernel<RT, LT, TOK, KS, GATED>, 200 * 1024);
+    cudaError_t e = ce_allow_smem(allowed, gemm_f32_stream_kernel<RT, LT, FIRST, TOK, KS, GATED>, 200 * 1024);
     if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_gemm_f32_stream: %s", cudaGetErrorString(e));
     ce_note("gemm_f32_stream_kernel");
-    ce_launch(gemm_f32_stream_kernel<RT, LT, TOK, KS, GATED>, (a.N + a.rows - 1) / a.rows, FS_THREADS, smem, stream, a);
+    ce_launch(gemm_f32_stream_kernel<RT, LT, FIRST, TOK, KS, GATED>, (a.N + a.rows - 1) / a.rows, FS_THREADS, smem, stream, a);
     return ce_check_launch("ce_gemm_f32_stream");
 }
 
-template <int RT, int LT, int KS>
-int fs_pick(const FsArgs& a, size_t smem, cudaStream_t stream) {
-    if (a.M <= 4) return GP_GATED(a.mode) ? fs_launch<RT, LT, 4, KS, true>(a, smem, stream) : fs_launch<RT, LT, 4, KS, false>(a, smem, stream);
-    return GP_GATED(a.mode) ? fs_launch<RT, LT, 8, KS, true>(a, smem, stream) : fs_launch<RT, LT, 8, KS, false>(a, smem, stream);
+template <int RT, int LT, int FIRST, int KS>
+int fs_pick(FsArgs a, bool shared_sm, cudaStream_t stream) {
+    const bool gated = GP_GATED(a.mode);
+    const int wrows = gated ? 2 * a.rows : a.rows, tok = a.M <= 4 ? 4 : 8;
+    a.stages = fs_stages(wrows, tok, KS);
+    size_t smem = a.stages * fs_stage_bytes(wrows, tok, KS);
+    if (smem > FS_MOST) return 1;
+    const size_t sums = sizeof(float) * FS_RUNS * tok * (size_t)(wrows + 1);
+    if (sums > smem) smem = sums;
+    if (!shared_sm && smem < FS_ALONE) smem = FS_ALONE;
+    if (tok == 4) return gated ? fs_launch<RT, LT, FIRST, 4, KS, true>(a, smem, stream) : fs_launch<RT, LT, FIRST, 4, KS, false>(a, smem, stream);
+    return gated ? fs_launch<RT, LT, FIRST, 8, KS, true>(a, smem, stream) : fs_launch<RT, LT, FIRST, 8, KS, false>(a, smem, stream);
 }
 
 }  // namespace
 
 // The product of ce_gemm_plain in float32, where this kernel takes its sizes: returns 1 where it does not, else as the other launchers.
 // It takes up to 8 tokens, K of eight equal runs (multiples of 32) on 16-byte rows, and as many rows as leave a ring of three stages.
+// Over 4 to 125 rows a block, 1 to 8 tokens and K of 2,048 to 12,288 it is the faster one but for the rule below.
 extern "C" int ce_gemm_f32_stream(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldc, int mode, const float* bias,
                                   float limit, float alpha, int weights_ready, cudaStream_t stream) {
     if (M < 1 || M > 8 || K < 2048 || K % 256 || lda % 4 || (((uintptr_t)A | (uintptr_t)W) & 15) || mode < GP_STORE || mode > GP_CLAMPGLU) return 1;
-    if (!A || !W || !C || N < 4 * FS_BLOCKS) return 1;
-    const int rows = (N + FS_BLOCKS - 1) / FS_BLOCKS, wrows = GP_GATED(mode) ? 2 * rows : rows, rt = (wrows + 31) / 32;
-    if (rt > 4) return 1;
-    const int tok = M <= 4 ? 4 : 8, ks = rt == 1 ? 32 : 16;
-    const size_t stage = sizeof(float) * FS_RUNS * (size_t)(wrows + tok) * ks;
-    // Eight stages where 150 KB hold them, else four, else three of what an SM has.  (14 rows and 4 tokens: eight stages, 147 KB, 1,433 us
-    // a pass of four decode steps of four layers; four stages, which leave room for the next product's block, 1,579.)
-    int stages = (int)(150 * 1024 / stage);
-    if (stages < 4) stages = (int)(196 * 1024 / stage);
-    if (stages < 3) return 1;
-    stages = stages >= 8 ? 8 : stages >= 4 ? 4 : 3;
-    size_t smem = stages * stage;
-    const size_t sums = sizeof(float) * FS_RUNS * tok * (size_t)(wrows + 1);
-    if (sums > smem) smem = sums;
-    FsArgs a{A, W, C, M, N, K, lda, ldc, mode, rows, stages, weights_ready, GpGate{bias, limit, alpha}};
-    if (wrows <= 16) return fs_pick<1, 2, 32>(a, smem, stream);
-    switch (rt) {
-        case 1: return fs_pick<1, 1, 32>(a, smem, stream);
-        case 2: return fs_pick<2, 1, 16>(a, smem, stream);
-        case 3: return fs_pick<3, 1, 16>(a, smem, stream);
-        default: return fs_pick<4, 1, 16>(a, smem, stream);
-    }
+    const int sms = ce_sm_count();
+    if (!A || !W || !C || N < 4 * sms) return 1;
+    const int rows = (N + sms - 1) / sms, blocks = (N + rows - 1) / rows, wrows = GP_GATED(mode) ? 2 * rows : rows;
+    FsArgs a{A, W, C, M, N, K, lda, ldc, mode, rows, 0, weights_ready, GpGate{bias, limit, alpha}};
+    // Up to 48 clusters of the other kernel run side by side, each near the memory's rate; 33 to 41 rows a block here cost nearly as much as 48.
+    // (4,884 rows, 1 token: K of 2,048 10.0 us there and 9.1 here, of 12,288 44.7 and 42.3; 5 to 8 tokens 13.3 and 12.7, but 61.9 and 63.5; gated,
+    // 2,516 features of 4,096: 16.9 and 17.7.)
+    const int tile = GP_GATED(mode) ? 64 : 128;
+    if (wrows > 32 && (N + tile - 1) / tile <= 48 && (GP_GATED(mode) || (M > 4 && K > 2048))) return 1;
+    // One block an SM where some SMs have none: the next product's blocks would take their places beside others and leave theirs empty
+    // (593 x 4,096, one product behind the other: 11.9 us with two blocks an SM, 8.4 with one).
+    const bool shared_sm = blocks == sms;
+    if (wrows <= 16) return fs_pick<1, 2, 4, 32>(a, shared_sm, stream);
+    if (wrows <= 32) return fs_pick<1, 1, 17, 32>(a, shared_sm, stream);
+    if (wrows <= 48) return fs_pick<3, 2, 33, 32>(a, shared_sm, stream);
+    if (wrows <= 64) return fs_pick<2, 1, 49, 16>(a, shared_sm, stream);
+    if (wrows <= 96) return fs_pick<3, 1, 65, 16>(a, shared_sm, stream);
+    if (wrows <= 128) return fs_pick<4, 1, 97, 16>(a, shared_sm, stream);
+    return 1;
 }

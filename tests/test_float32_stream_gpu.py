@@ -33,3 +33,13 @@ def test_stream_products_have_the_bits_of_the_tiles(N, K, gated, M, weights_read
         [(ops.GEMM_STORE, None), (ops.GEMM_ACCUM_F32, None), (ops.GEMM_RELU2, None)]
     for mode, glu in modes:
         assert torch.equal(run(a[7:7 + M], mode, glu), run(a, mode, glu)[7:7 + M]), mode
+
+
+# every depth of a ring that a number of rows can have (a block's rows, then stages for 1 to 4 and 5 to 8 tokens): 8 / 8 and 6 (7, 16 rows),
+# 7 / 6 (17), 5 / 4 (26), 4 / 4 (33, 45: three rows a lane, two groups of lanes), 6 / 5 (49), 5 / 4 (60), 4 / 3 (66, 90), 3 / - (100)
+@pytest.mark.parametrize("N,K,gated", [(890, 2304, False), (2367, 2048, False), (2500, 2304, False), (3700, 2048, False), (6300, 2304, False),
+                                       (6660, 2816, False), (7201, 2048, False), (8879, 2304, False), (9700, 2048, False), (13300, 2048, False),
+                                       (14700, 2048, False), (1190, 2048, True), (1340, 2304, True), (3300, 2816, True), (3552, 2048, True)])
+@pytest.mark.parametrize("M", [1, 8])
+def test_rings_of_every_depth_have_the_bits_of_the_tiles(N, K, gated, M):
+    test_stream_products_have_the_bits_of_the_tiles(N, K, gated, M, True)

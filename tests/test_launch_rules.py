@@ -27,7 +27,7 @@ def linked(tmp_path_factory):
         pytest.skip("no CUDA toolkit")
     cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
     headers = build._sources(build.KERNEL_DIR, (".cuh", ".h"))
-    names = ("errors", "tensor_map", "gemm_tc", "gemm_f32", "gemm_plain", "attention_f32", "attention_mma")
+    names = ("errors", "tensor_map", "gemm_tc", "gemm_f32", "gemm_f32_stream", "gemm_plain", "attention_f32", "attention_mma")
     objects = build._compile_all(nvcc, build.NVCC_FLAGS, [os.path.join(build.KERNEL_DIR, n + ".cu") for n in names], headers, build.build_dir(), "k")
     out = str(tmp_path_factory.mktemp("fake") / "libfake.so")
     cxx = os.environ.get("CXX") or shutil.which("g++") or shutil.which("c++")
@@ -64,6 +64,16 @@ class Chip:
     def gemm_f32(self, M, N, K, mode=STORE, weights_ready=1):
         p = ctypes.c_void_p(ADDR)
         return self._launched(self.lib.ce_gemm_plain(p, p, p, 0, M, N, K, K, N, mode, None, ctypes.c_float(0), ctypes.c_float(0), weights_ready, None))
+
+    def stream(self, M, N, K, mode=STORE, lda=None, at=ADDR):
+        """The product of a few tokens as a stream of weights; None where the launcher leaves it to the other kernel."""
+        p, w = ctypes.c_void_p(at), ctypes.c_void_p(ADDR)
+        before = self.lib.fake_launches()
+        code = self.lib.ce_gemm_f32_stream(p, w, w, M, N, K, K if lda is None else lda, N, mode, None, ctypes.c_float(0), ctypes.c_float(0), 1, None)
+        if code == 1:
+            assert self.lib.fake_launches() == before
+            return None
+        return self._launched(code)
 
     def attention_f32(self, n_decode, n_tiles, heads=16, kv_heads=4, d=128, longest=4096):
         p = ctypes.c_void_p(ADDR)
@@ -166,6 +176,48 @@ def test_heads_of_192_and_256_are_asked_for_apart(linked):
     for d in (192, 256, 192, 256):
         chip.decode(1, 2304, d=d)
     assert chip.lib.fake_occupancy_calls() == 2
+
+
+def ring(rows, tokens, k):
+    """Bytes of one stage: eight warps with the rows and tokens of a block."""
+    return 8 * 4 * (rows + tokens) * k
+
+
+# a block's rows, tokens (rounded up to 4 or 8), k and number of a ring's stages
+@pytest.mark.parametrize("M,N,K,mode,rows,tokens,k,stages", [
+    (1, 2048, 2048, STORE, 14, 4, 32, 8), (4, 2048, 6144, ACCUM, 14, 4, 32, 8), (8, 2048, 2048, STORE, 14, 8, 32, 6), (5, 2368, 2048, STORE, 16, 8, 32, 6),
+    (4, 2516, 2560, STORE, 17, 4, 32, 7), (4, 2560, 9728, ACCUM, 18, 4, 32, 6), (8, 2560, 9728, ACCUM, 18, 8, 32, 5), (1, 3072, 2048, STORE, 21, 4, 32, 6),
+    (4, 4096, 4096, ACCUM, 28, 4, 32, 4), (3, 5120, 5120, ACCUM, 35, 4, 32, 4), (4, 7104, 2048, STORE, 48, 4, 32, 3), (4, 7168, 5120, STORE, 49, 4, 16, 5),
+    (4, 6144, 2048, SWIGLU, 84, 4, 16, 4), (8, 6144, 2048, SWIGLU, 84, 8, 16, 4), (8, 8140, 2048, SWIGLU, 110, 8, 16, 3), (2, 1184, 2304, CLAMPGLU, 16, 4, 32, 7)])
+def test_a_streamed_products_ring_takes_all_stages_that_fit(linked, M, N, K, mode, rows, tokens, k, stages):
+    seen = Chip(linked, {}).stream(M, N, K, mode)
+    blocks = -(-N * (2 if mode >= SWIGLU else 1) // rows)
+    assert b"gemm_f32_stream_kernel" in seen.kernel and seen.dependent and seen.grid[0] == blocks
+    assert seen.smem == max(stages * ring(rows, tokens, k), 116 * 1024 if blocks < 148 else 0)
+
+
+def test_streamed_products_fit_every_device(linked):
+    """All numbers of rows: the opt-in on each device of a process, and no more shared memory than an SM has."""
+    chip = Chip(linked, {})
+    taken = set()
+    for device, (M, mode) in enumerate([(4, STORE), (8, STORE), (4, SWIGLU), (8, CLAMPGLU), (1, ACCUM)]):
+        chip.lib.fake_device(device)
+        for rows in range(4, 140):
+            seen = chip.stream(M, 148 * rows, 2048, mode)
+            if seen:
+                taken.add((M, mode, rows))
+                assert seen.device == device and seen.grid[0] == 148 and seen.smem <= 200 * 1024
+    assert max(r for M, mode, r in taken if (M, mode) == (4, STORE)) == 126 and max(r for M, mode, r in taken if (M, mode) == (8, CLAMPGLU)) == 61
+
+
+@pytest.mark.parametrize("M,N,K,mode,lda,at", [
+    (0, 2048, 2048, STORE, None, ADDR), (9, 2048, 2048, STORE, None, ADDR), (4, 591, 2048, STORE, None, ADDR), (4, 2048, 1792, STORE, None, ADDR),
+    (4, 2048, 2080, STORE, None, ADDR), (4, 2048, 2048, STORE, 2050, ADDR), (4, 2048, 2048, STORE, None, ADDR + 4), (4, 2048, 2048, STORE, None, 0),
+    (4, 2048, 2048, 7, None, ADDR), (4, 2048, 2048, -1, None, ADDR), (1, 151936, 2048, STORE, None, ADDR), (4, 9728, 2560, SWIGLU, None, ADDR),
+    # 33 to 41 rows a block, where the tiles' clusters run side by side: gated ones, and more than 4 tokens beyond K = 2,048
+    (4, 2960, 4096, SWIGLU, None, ADDR), (8, 5120, 5120, ACCUM, None, ADDR), (5, 6144, 4096, STORE, None, ADDR)])
+def test_products_that_are_not_streamed(linked, M, N, K, mode, lda, at):
+    assert Chip(linked, {}).stream(M, N, K, mode, lda, at) is None
 
 
 def test_without_room_for_a_cluster_the_float32_kernels_run_without(linked):
