@@ -553,6 +553,16 @@ __device__ __forceinline__ void warp_tile_swz(const uint32_t (&qf)[DMAX / 16][2]
     }
 }
 
+// Tiles of a block of a cluster: the sequence's own in equal shares (blocks from ceil(tiles / share) on stay idle), since shares cut from the
+// batch's longest context leave a sequence of half that length to half of its cluster's blocks; but the shares of the longest context where equal ones
+// would be less than a tenth shorter: the last block then ends early and lets the next kernel's blocks in.  (Eight steps of 12 layers, 8
+// sequences of 2,048 keys, 33 tiles: 11,183 us as 10, 10, 10 and 3 tiles, 11,224 as 9, 9, 9 and 6.)
+__host__ __device__ inline int decode_share(int tiles, int splits, int longest_share) {
+    const int even = (tiles + splits - 1) / splits;
+    return 10 * even < 9 * longest_share || even > longest_share ? even : longest_share;
+}
+extern "C" int ce_attention_decode_share(int tiles, int splits, int longest_share) { return decode_share(tiles, splits, longest_share); }
+
 template <int DMAX, int ST, bool BIAS>
 __global__ void __launch_bounds__(AMT_THREADS) attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k,
                                                                           const __grid_constant__ CUtensorMap map_v,
@@ -569,7 +579,8 @@ __global__ void __launch_bounds__(AMT_THREADS) attention_decode_tma_kernel(const
     int G = a.nh / a.nkv;
     if (a.longest_first) {
         // Clusters start in the order of their numbers, as room becomes free: sequences with the most keys first (all KV heads of one,
-        // then the next), so that the last to start are the shortest.  The order is taken from the positions, which are there anyway.
+        // then the next), so that the last to start are the shortest (with more than 8 heads a KV head each group of 8, a blockIdx.z, has this
+        // order for itself: the groups start one after the other).  The order is taken from the positions, which are there anyway.
         // (21 sequences of 450 to 9,000 keys, 8 KV heads, a pass of four steps of 12 layers: 10.42 ms as the batch has them, cut at shares of
         // the longest context; 10.46 with the order alone, 9.51 with a sequence's own shares alone, 8.33 with both, 8.56 since such a grid stands alone.)
         __shared__ __align__(16) int s_pos[AMT_MAX_SORTED];
@@ -597,9 +608,7 @@ __global__ void __launch_bounds__(AMT_THREADS) attention_decode_tma_kernel(const
     int k_begin, k_end;
     bool idle;
     if (a.cluster_merge) {
-        // the sequence's own tiles, in equal shares but for the last block's (shares cut from the batch's longest context leave a sequence
-        // of half that length to half of its cluster's blocks)
-        const int tile0 = lo / AM_TILE, tiles_seq = pos / AM_TILE + 1 - tile0, share = (tiles_seq + a.max_splits - 1) / a.max_splits;
+        const int tile0 = lo / AM_TILE, share = decode_share(pos / AM_TILE + 1 - tile0, a.max_splits, a.split / AM_TILE);
         k_begin = (tile0 + split * share) * AM_TILE;
         k_end = min(k_begin + share * AM_TILE, pos + 1);
         idle = k_begin >= k_end;                 // the merge skips it
@@ -1094,7 +1103,8 @@ extern "C" int ce_attention_decode_bf16_sink(const void* q, const void* k_pool, 
     // inside a cluster (at most 8 of them) or, where that leaves most of the GPU idle (one sequence with a
     // long context: 8 KV heads x 8 splits are 64 blocks), through scratch memory and a merge kernel, whose
     // launch is worth about six tiles more.  The choice depends on the number of one-token sequences and on
-    // max_splits, not on their contents.  (In a cluster a sequence's own tiles are then dealt to that many blocks evenly.)
+    // max_splits, not on their contents: the model counts every sequence as the longest (in a cluster decode_share deals a sequence's
+    // own tiles to that many blocks).
     bool use_cluster = false;
     {
         long long pairs = (long long)n_seqs * nkv * ((G + hgroup - 1) / hgroup);
@@ -1105,7 +1115,7 @@ extern "C" int ce_attention_decode_bf16_sink(const void* q, const void* k_pool, 
             int splits = (max_splits + m - 1) / m;
             long long blocks = pairs * splits;
             // a block's fixed cost in tiles' worth of time.  The bound the splits are cut from is rounded up to a bucket
-            // (one captured graph per bucket), so a sequence's last split is part empty; with a small fixed cost the
+            // (one captured graph per bucket), so the last split of the longest sequence is part empty; with a small fixed cost the
             // model cut many sequences in two unequal splits where one block a sequence is faster.  Measured with 6 /
             // 10 / 14 units, ms a step: batch 128 at 2,048 tokens 12.34 / 11.66 / 11.65, batch 64 at 8,192 17.54 /
             // 15.97 / 15.98, batch 8 at 32,768 9.57 / 9.57 / 9.03; batch 1 to 64 at 2,048 and batch 1 at 32,768 the same.
