@@ -70,7 +70,6 @@ struct MmaAttnArgs {
     int* counters;              // decode: one per (sequence, KV head, head group), zero between launches
     int* status;
     int nh, nkv, d, q_stride, page_size, max_pages, num_pages, window, max_splits, split, fused_merge;
-    int longest_first;          // TMA decode kernel: clusters take the sequences by their lengths, the longest first
     int overlap;                // TMA decode kernel: kernels behind may start before this one ends
     int cluster_merge;          // TMA decode kernel: the splits of a sequence form a cluster and merge through shared memory
     float scale_log2;           // scale * log2(e)
@@ -563,7 +562,8 @@ __host__ __device__ inline int decode_share(int tiles, int splits, int longest_s
 }
 extern "C" int ce_attention_decode_share(int tiles, int splits, int longest_share) { return decode_share(tiles, splits, longest_share); }
 
-template <int DMAX, int ST, bool BIAS>
+// ORDER: clusters take the sequences by their lengths, the longest first
+template <int DMAX, int ST, bool BIAS, bool ORDER>
 __global__ void __launch_bounds__(AMT_THREADS) attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k,
                                                                           const __grid_constant__ CUtensorMap map_v,
                                                                           MmaAttnArgs a, int box_rows) {
@@ -576,34 +576,45 @@ __global__ void __launch_bounds__(AMT_THREADS) attention_decode_tma_kernel(const
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[ST], empty_bar[ST];
     int split = blockIdx.x % a.max_splits, b = blockIdx.x / a.max_splits, kvh = blockIdx.y, hg = blockIdx.z;
-    int G = a.nh / a.nkv;
-    if (a.longest_first) {
-        // Clusters start in the order of their numbers, as room becomes free: sequences with the most keys first (all KV heads of one,
-        // then the next), so that the last to start are the shortest (with more than 8 heads a KV head each group of 8, a blockIdx.z, has this
-        // order for itself: the groups start one after the other).  The order is taken from the positions, which are there anyway.
+    int G = a.nh / a.nkv, pos, slot;
+    if (ORDER) {
+        // Clusters start in the order of their numbers, as room becomes free: all KV heads of a sequence, whose rows lie side by side in a
+        // page, then the next one's; sequences with the most keys first, so that the last to start are the shortest (with more than 8 heads a
+        // KV head each group of 8, a blockIdx.z, has this order for itself: the groups start one after the other).  The order is taken from
+        // the positions, which are there anyway, by every block for itself, which costs it up to a microsecond (128 sequences): not where
+        // all lengths are about the first's.
         // (21 sequences of 450 to 9,000 keys, 8 KV heads, a pass of four steps of 12 layers: 10.42 ms as the batch has them, cut at shares of
-        // the longest context; 10.46 with the order alone, 9.51 with a sequence's own shares alone, 8.33 with both, 8.56 since such a grid stands alone.)
+        // the longest context; 10.46 with the order alone, 9.51 with a sequence's own shares alone, 8.33 with both, 8.56 since such a grid stands
+        // alone.)
         __shared__ __align__(16) int s_pos[AMT_MAX_SORTED];
-        __shared__ int s_b;
+        __shared__ int s_slot[AMT_MAX_SORTED], s_b;
+        static_assert(AMT_MAX_SORTED <= AMT_THREADS, "a thread a sequence");
         const int n = gridDim.x / a.max_splits, at = blockIdx.y * n + b, rank = at / a.nkv;
-        for (int i = threadIdx.x; i < (n + 3) / 4 * 4; i += AMT_THREADS) s_pos[i] = i < n ? a.positions[i] : INT_MIN;
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += AMT_THREADS) {
-            // sequences in front: those with more keys, and of those with as many the ones before it
-            const int mine = s_pos[i];
-            int before = 0;
-            for (int j = 0; j < n; j += 4) {
-                const int4 p = *reinterpret_cast<const int4*>(s_pos + j);
-                before += (p.x >= mine + (j >= i)) + (p.y >= mine + (j + 1 >= i)) + (p.z >= mine + (j + 2 >= i)) + (p.w >= mine + (j + 3 >= i));
-            }
-            if (before == rank) s_b = i;
-        }
-        __syncthreads();
-        b = s_b;
+        const int i = threadIdx.x, mine = i < n ? a.positions[i] : INT_MIN, first = a.positions[0];
+        if (i < (n + 3) / 4 * 4) s_pos[i] = mine;
+        if (i < n) s_slot[i] = a.seq_slot[i];
+        b = rank;
         kvh = at - rank * a.nkv;
+        if (__syncthreads_or(i < n && abs(mine - first) > first / 8)) {
+            if (i < n) {
+                // sequences in front: those with more keys, and of those with as many the ones before it
+                int before = 0;
+                for (int j = 0; j < n; j += 4) {
+                    const int4 p = *reinterpret_cast<const int4*>(s_pos + j);
+                    before += (p.x >= mine + (j >= i)) + (p.y >= mine + (j + 1 >= i)) + (p.z >= mine + (j + 2 >= i)) + (p.w >= mine + (j + 3 >= i));
+                }
+                if (before == rank) s_b = i;
+            }
+            __syncthreads();
+            b = s_b;
+        }
+        pos = s_pos[b];
+        slot = s_slot[b];
+    } else {
+        pos = a.positions[b];
+        slot = a.seq_slot[b];
     }
     int t = b;
-    int pos = a.positions[t];
     int lo = a.window > 0 ? max(0, pos - a.window + 1) : 0;
     int k_begin, k_end;
     bool idle;
@@ -619,7 +630,7 @@ __global__ void __launch_bounds__(AMT_THREADS) attention_decode_tma_kernel(const
         k_begin = max(k_begin, lo / AM_TILE * AM_TILE);      // whole tiles below the window are not even looked up
     }
     if (idle && !a.cluster_merge) return;
-    const int* table = a.block_table + (size_t)a.seq_slot[b] * a.max_pages;
+    const int* table = a.block_table + (size_t)slot * a.max_pages;
     int d = a.d, panels = d >> 6;
     uint32_t base = (amt_smem(smem_raw) + 1023u) & ~1023u;        // the swizzle is keyed on address bits
     unsigned char* tiles = smem_raw + (base - amt_smem(smem_raw));
@@ -996,10 +1007,14 @@ template <typename F> static int set_smem(F kernel, size_t bytes, const char* wh
 
 // One launch of the TMA decode kernel.  Clusters stand alone where there are more of them than the chip holds (ce_clusters_at_once):
 // 21 sequences x 8 KV heads of up to 9,000 keys are 168 clusters of 3 where 93 have room (a pass of four steps of 12 layers 8.41 -> 8.56 ms).
+// The longest sequences come first in grids of one to two waves whose blocks have work enough (one launch of 64 sequences of 30 to 600 keys
+// 28.8 -> 26.0 us, of 100 to 2,000 65.2 -> 55.0): in one wave none is the last to start (32 sequences of 300 keys: 11.1, in order 11.7), with
+// more waves the ends even out by themselves (128 of 30 to 600: 51.6, in order 57.7), and short blocks pay for taking the order (64 of
+// 128 keys: 15.8, in order 17.0).
 template <int DM, int ST, bool BIAS>
 static int launch_decode_tma(const CUtensorMap& mk, const CUtensorMap& mv, MmaAttnArgs a, int box_rows, dim3 grid, size_t smem, cudaStream_t stream) {
-    int rc = set_smem(attention_decode_tma_kernel<DM, ST, BIAS>, smem, "ce_attention_decode_bf16");
-    if (rc) return rc;
+    int rc = set_smem(attention_decode_tma_kernel<DM, ST, BIAS, false>, smem, "ce_attention_decode_bf16");
+    if (rc || (rc = set_smem(attention_decode_tma_kernel<DM, ST, BIAS, true>, smem, "ce_attention_decode_bf16"))) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(AMT_THREADS);
@@ -1008,20 +1023,23 @@ static int launch_decode_tma(const CUtensorMap& mk, const CUtensorMap& mv, MmaAt
     cudaLaunchAttribute attr[2];
     cfg.attrs = attr;
     a.overlap = 1;
+    bool order = false;
     if (a.cluster_merge) {
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = a.max_splits; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
         cfg.numAttrs = 1;
         static CeRoom room[2][9];                       // (heads of 192 and of 256 share an instantiation, not their shared memory)
-        if (a.max_splits > 1)
-            a.overlap = (long long)grid.x / a.max_splits * grid.y * grid.z <=
-                        ce_clusters_at_once(room[a.d == DM][a.max_splits], attention_decode_tma_kernel<DM, ST, BIAS>, cfg);
+        const int at_once = ce_clusters_at_once(room[a.d == DM][a.max_splits], attention_decode_tma_kernel<DM, ST, BIAS, true>, cfg);
+        const long long n_seqs = grid.x / a.max_splits, clusters = n_seqs * grid.y * grid.z;
+        a.overlap = a.max_splits == 1 || clusters <= at_once;
+        order = n_seqs > 1 && n_seqs <= AMT_MAX_SORTED && clusters > at_once && clusters <= 2LL * at_once && (long long)a.split * a.d >= 512 * 128;
     }
     if (a.overlap && ce_pdl_enabled()) {
         attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, attention_decode_tma_kernel<DM, ST, BIAS>, mk, mv, a, box_rows);
+    const cudaError_t e = order ? cudaLaunchKernelEx(&cfg, attention_decode_tma_kernel<DM, ST, BIAS, true>, mk, mv, a, box_rows)
+                                : cudaLaunchKernelEx(&cfg, attention_decode_tma_kernel<DM, ST, BIAS, false>, mk, mv, a, box_rows);
     if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_attention_decode_bf16: %s", cudaGetErrorString(e));
     return ce_check_launch("ce_attention_decode_bf16");
 }
@@ -1152,7 +1170,6 @@ extern "C" int ce_attention_decode_bf16_sink(const void* q, const void* k_pool, 
         if (comb > tsmem) tsmem = comb;
         tsmem += 1024;
         a.cluster_merge = use_cluster;
-        a.longest_first = use_cluster && n_seqs > 1 && n_seqs <= AMT_MAX_SORTED;
         ce_note(a.cluster_merge ? "attention_decode_tma_kernel (merge in the cluster)" : "attention_decode_tma_kernel");
         // three stages for heads of up to 128 (deep3), two above
 #define AMT_LAUNCH(DM, ST)                                                                              \

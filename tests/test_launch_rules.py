@@ -173,10 +173,20 @@ def test_a_sequences_tiles_are_dealt_evenly_unless_it_is_about_the_longest(linke
     assert share * blocks >= tiles                                   # nothing is left out
 
 
+# clusters at once of the B200 measured, heads of 128: sequences, longest context, room; 8 KV heads
+@pytest.mark.parametrize("n,longest,d,room,ordered", [
+    (21, 9000, 128, {3: 93}, True), (64, 700, 128, {1: 296}, True), (48, 700, 128, {1: 296}, True),
+    (37, 700, 128, {1: 296}, False), (38, 700, 128, {1: 296}, True), (74, 700, 128, {1: 296}, True), (75, 700, 128, {1: 296}, False),      # one and two waves
+    (64, 384, 128, {1: 296}, False), (64, 512, 128, {1: 296}, True), (100, 890, 64, {1: 592}, False), (100, 1000, 64, {1: 592}, True),   # work of a block
+    (128, 2048, 64, {1: 592}, True), (129, 2048, 64, {1: 592}, False), (8, 2304, 128, {4: 71}, False)])
+def test_decode_attention_takes_the_longest_first_in_grids_of_one_to_two_waves(linked, n, longest, d, room, ordered):
+    seen = Chip(linked, room).decode(n, longest, d=d)
+    assert (f"attention_decode_tma_kernelILi{d}ELi3ELb0ELb{int(ordered)}E".encode()) in seen.kernel
+
+
 def test_decode_attention_of_one_block_a_sequence_overlaps(linked):
-    chip = Chip(linked, {1: 1})
-    seen = chip.decode(64, 2304)
-    assert seen.cluster[0] == 1 and seen.dependent and chip.lib.fake_occupancy_calls() == 0
+    seen = Chip(linked, {1: 1}).decode(64, 2304)
+    assert seen.cluster[0] == 1 and seen.dependent
 
 
 def test_heads_of_192_and_256_are_asked_for_apart(linked):

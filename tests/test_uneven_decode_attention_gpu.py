@@ -47,10 +47,14 @@ def decode(lens, nh, nkv, d, ps, window, scale, sinks, out_scale, slopes, seed):
         vp[table[i].long()[at // ps], :, at % ps] = v
         q_step[i, :nh * d] = q.reshape(-1)
         k, v = k.double().repeat_interleave(nh // nkv, 1), v.double().repeat_interleave(nh // nkv, 1)
-        s = torch.einsum("hd,lhd->hl", q.double(), k) * scale - slopes.double()[:, None] * (L - 1 - at)
+        s = torch.einsum("hd,lhd->hl", q.double(), k) * scale
+        if slopes is not None:
+            s = s - slopes.double()[:, None] * (L - 1 - at)
         if window:
             s = s.masked_fill(L - 1 - at >= window, float("-inf"))
-        p = torch.softmax(torch.cat([s, sinks.double()[:, None]], 1), 1)[:, :L]
+        if sinks is not None:
+            s = torch.cat([s, sinks.double()[:, None]], 1)
+        p = torch.softmax(s, 1)[:, :L]
         want[i] = torch.einsum("hl,lhd->hd", p, v) * out_scale
     out = torch.full((len(lens), nh * d), float("nan"), dtype=torch.bfloat16, device=dev())
     assert ops_tensor.attention_bf16(ctx, ctx, q_step, out, FakeCache(kp, vp, ps), table, nh, nkv, d, window, scale, sinks, out_scale, slopes)
@@ -74,3 +78,18 @@ def test_many_heads_a_group_with_sinks_and_a_penalty_on_distance(n, nh, nkv, d, 
     again, _ = decode([lens[i] for i in order], nh, nkv, d, ps, window, 1 / math.sqrt(d), sinks, 0.8, slopes, 3)
     for at, i in enumerate(order):
         assert torch.equal(again[at], got[i]), (i, lens[i])
+
+
+# Grids of one to two waves, whose clusters take the longest sequences first (of one, three and two blocks), and one of one wave: unequal
+# contexts, and contexts that are about the same, where the batch's order stays
+@pytest.mark.parametrize("n,nh,nkv,d,longest", [(64, 8, 8, 128, 700), (21, 8, 8, 128, 9000), (100, 8, 8, 64, 1200), (48, 8, 8, 64, 4000), (30, 8, 8, 256, 300),
+                                                (128, 16, 8, 64, 1030), (5, 40, 10, 192, 6000)])
+@pytest.mark.parametrize("spread", [0.95, 0.1])
+def test_the_longest_first(n, nh, nkv, d, longest, spread):
+    lens = [max(1, round(longest * (1 - spread * ((i * 37) % n) / n))) for i in range(n)]
+    got, want = decode(lens, nh, nkv, d, 16, 0, 1 / math.sqrt(d), None, 1.0, None, 5)
+    for i in range(n):
+        assert rel_err(got[i], want[i]) < 2e-2, (i, lens[i])
+    order = sorted(range(n), key=lambda i: (i * 11) % n)
+    again, _ = decode([lens[i] for i in order], nh, nkv, d, 16, 0, 1 / math.sqrt(d), None, 1.0, None, 5)
+    assert torch.equal(again, got[order])
