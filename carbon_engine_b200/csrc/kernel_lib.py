@@ -94,8 +94,9 @@ _SIGNATURES = {
     # q, k_pool, v_pool, out, positions, seq_slot, q_start, block_table, tiles, status,
     # n_decode, n_tiles, nh, nkv, d, q_stride, page_size, max_pages, num_pages, window, max_ctx, scale, stream
     "ce_attention_f32": (_i, [_p] * 10 + [_i] * 11 + [_f, _p]),
-    # A, W, C, dtype, M, N, K, lda, ldc, mode, bias, limit, alpha, weights_ready, stream
+    # A, W, C, M, N, K, lda, ldc, mode, bias, limit, alpha, weights_ready, stream (1: not sizes of this kernel)
     "ce_gemm_f32_stream": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _i, _p, _f, _f, _i, _p]),
+    # A, W, C, dtype, M, N, K, lda, ldc, mode, bias, limit, alpha, weights_ready, stream
     "ce_gemm_plain": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _p, _f, _f, _i, _p]),
     "ce_sample": (_i, [_p, _i, _i, _p, _p, _p]),
     "ce_argmax": (_i, [_p, _i, _i, _p, _p]),

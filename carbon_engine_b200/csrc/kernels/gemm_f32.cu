@@ -13,9 +13,12 @@
 // or 4 tokens where a thread holds one weight row and all tokens, whose values are broadcast reads.  Operands come by cp.async into
 // a ring of stages of 32 k, rows as they lie in memory with 16-byte chunks swizzled by the row (chunk ^ row & 7), so that the lanes'
 // reads meet no bank twice.  Where a product has too few tiles to fill the chip, a cluster of blocks takes a run of K each and adds
-// the partial sums through distributed shared memory, in the order above.
+// the partial sums through distributed shared memory, in the order above.  Most products of up to 8 tokens with K of 2,048 and more go to
+// gemm_f32_stream.cu instead (the same bits); the small tiles here take the others: shorter or odd K, rows off 16 bytes, few or very many
+// weight rows (the vocabulary's, whose clusters are more than the chip holds at once).
 //
-// Measured (us; before: 64 x 64 tiles, 4 x 4 results a thread, one stage of 16 k, one block a tile over all of K):
+// Measured (us; 1 and 8 tokens of these two go to gemm_f32_stream.cu now; before: 64 x 64 tiles, 4 x 4 results a thread, one stage of 16 k,
+// one block a tile over all of K):
 //                          12,288 x 2,048 (gate and up)      2,048 x 6,144 (down)
 //     1 token                  485 -> 22 (4.5 TB/s)             985 -> 18
 //     8 tokens                 495 -> 28                        987 -> 28

@@ -6,9 +6,10 @@ products (src/model/attention.rs:871).  The epilogue is part of the product: sto
 activation dtype, store float32 (logits), add into the float32 residual stream, or a gated activation
 (SiLU or ReLU of the gate rows times the up rows).
 
-float32 runs FMA arithmetic only (gemm_f32.cu).  bfloat16 runs the tensor-core kernels of
-``csrc/kernels`` when they accept the shape and otherwise a library product (cuBLAS through
-``torch.matmul``, where the reference also calls a library) followed by the epilogue kernel.
+float32 runs FMA arithmetic only (gemm_f32.cu; most products of up to 8 tokens gemm_f32_stream.cu, with the
+same bits).  bfloat16 runs the tensor-core kernels of ``csrc/kernels`` when they accept the shape and
+otherwise a library product (cuBLAS through ``torch.matmul``, where the reference also calls a library)
+followed by the epilogue kernel.
 """
 from __future__ import annotations
 

@@ -99,7 +99,7 @@ def step_meta(seqs):
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("nh,nkv,d,rd,ps", [(6, 3, 48, 48, 8), (4, 1, 16, 16, 16), (5, 5, 80, 32, 4), (2, 2, 256, 256, 64),
                                             (8, 2, 128, 128, 64), (3, 1, 64, 64, 16), (4, 2, 192, 192, 8), (2, 1, 128, 64, 16)])
-@pytest.mark.parametrize("first", [9, 270])        # few tokens: a warp a head; from 256 tokens on a warp takes several heads of a token
+@pytest.mark.parametrize("first", [9, 270])        # (from 256 tokens on a warp takes a quarter of a token's heads)
 def test_qk_norm_rope_and_cache_write(ops, dtype, nh, nkv, d, rd, ps, first):
     torch.manual_seed(1)
     seqs = [(5, first), (0, 3), (30, 1)]
