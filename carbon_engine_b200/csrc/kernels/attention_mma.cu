@@ -1013,8 +1013,11 @@ template <typename F> static int set_smem(F kernel, size_t bytes, const char* wh
 // 128 keys: 15.8, in order 17.0).
 template <int DM, int ST, bool BIAS>
 static int launch_decode_tma(const CUtensorMap& mk, const CUtensorMap& mv, MmaAttnArgs a, int box_rows, dim3 grid, size_t smem, cudaStream_t stream) {
-    int rc = set_smem(attention_decode_tma_kernel<DM, ST, BIAS, false>, smem, "ce_attention_decode_bf16");
-    if (rc || (rc = set_smem(attention_decode_tma_kernel<DM, ST, BIAS, true>, smem, "ce_attention_decode_bf16"))) return rc;
+    static std::atomic<unsigned long long> allowed[2];
+    constexpr int most = ST * 2 * (DM / 64) * 8192 + 1024;                 // (the largest head size of the instantiation)
+    cudaError_t e = ce_allow_smem(allowed[0], attention_decode_tma_kernel<DM, ST, BIAS, false>, most);
+    if (e == cudaSuccess) e = ce_allow_smem(allowed[1], attention_decode_tma_kernel<DM, ST, BIAS, true>, most);
+    if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_attention_decode_bf16: %s", cudaGetErrorString(e));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(AMT_THREADS);
@@ -1038,8 +1041,8 @@ static int launch_decode_tma(const CUtensorMap& mk, const CUtensorMap& mv, MmaAt
         attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
-    const cudaError_t e = order ? cudaLaunchKernelEx(&cfg, attention_decode_tma_kernel<DM, ST, BIAS, true>, mk, mv, a, box_rows)
-                                : cudaLaunchKernelEx(&cfg, attention_decode_tma_kernel<DM, ST, BIAS, false>, mk, mv, a, box_rows);
+    e = order ? cudaLaunchKernelEx(&cfg, attention_decode_tma_kernel<DM, ST, BIAS, true>, mk, mv, a, box_rows)
+              : cudaLaunchKernelEx(&cfg, attention_decode_tma_kernel<DM, ST, BIAS, false>, mk, mv, a, box_rows);
     if (e != cudaSuccess) return ce_fail(CE_ERR_CUDA, "ce_attention_decode_bf16: %s", cudaGetErrorString(e));
     return ce_check_launch("ce_attention_decode_bf16");
 }

@@ -128,10 +128,12 @@ def test_float32_products_of_few_tiles_give_each_block_of_a_cluster_a_run_of_k(l
 
 
 @pytest.mark.parametrize("launch", [lambda c: c.gemm_f32(100, 4096, 4096), lambda c: c.attention_f32(0, 40), lambda c: c.gemm_tc(4, 4096, 4096),
-                                    lambda c: c.gemm_tc(200, 4096, 4096), lambda c: c.gemm_tc(2048, 4096, 4096), lambda c: c.gemm_tc(2048, 128, 4096)],
-                         ids=["float32 product", "float32 attention", "one-block product", "shared pairs", "pairs", "single CTAs"])
+                                    lambda c: c.gemm_tc(200, 4096, 4096), lambda c: c.gemm_tc(2048, 4096, 4096), lambda c: c.gemm_tc(2048, 128, 4096),
+                                    lambda c: c.decode(64, 700), lambda c: c.decode(64, 300), lambda c: c.decode(64, 300, d=192), lambda c: c.decode(64, 300, d=256)],
+                         ids=["float32 product", "float32 attention", "one-block product", "shared pairs", "pairs", "single CTAs", "decode attention, longest first",
+                              "decode attention", "decode attention, heads of 192", "decode attention, heads of 256"])
 def test_kernels_of_much_shared_memory_run_on_every_device_of_a_process(linked, launch):
-    chip = Chip(linked, B200)
+    chip = Chip(linked, {1: 296, **B200})
     for device in (0, 1, 0, 70, 71):
         chip.lib.fake_device(device)
         seen = launch(chip)
