@@ -70,6 +70,7 @@ struct MmaAttnArgs {
     int* counters;              // decode: one per (sequence, KV head, head group), zero between launches
     int* status;
     int nh, nkv, d, q_stride, page_size, max_pages, num_pages, window, max_splits, split, fused_merge;
+    int longest_share;          // TMA decode kernel: see decode_share
     int overlap;                // TMA decode kernel: kernels behind may start before this one ends
     int cluster_merge;          // TMA decode kernel: the splits of a sequence form a cluster and merge through shared memory
     float scale_log2;           // scale * log2(e)
@@ -555,7 +556,8 @@ __device__ __forceinline__ void warp_tile_swz(const uint32_t (&qf)[DMAX / 16][2]
 // Tiles of a block of a cluster: the sequence's own in equal shares (blocks from ceil(tiles / share) on stay idle), since shares cut from the
 // batch's longest context leave a sequence of half that length to half of its cluster's blocks; but the shares of the longest context where equal ones
 // would be less than a tenth shorter: the last block then ends early and lets the next kernel's blocks in.  (Eight steps of 12 layers, 8
-// sequences of 2,048 keys, 33 tiles: 11,183 us as 10, 10, 10 and 3 tiles, 11,224 as 9, 9, 9 and 6.)
+// sequences of 2,048 keys, 33 tiles: 11,183 us as 10, 10, 10 and 3 tiles, 11,224 as 9, 9, 9 and 6.)  Nothing is let in by a grid of more blocks
+// than the chip takes at once, which gives longest_share 0 (20 sequences of 600 to 6,000 keys, one launch: 58.8 us, with the longest's shares 61.0).
 __host__ __device__ inline int decode_share(int tiles, int splits, int longest_share) {
     const int even = (tiles + splits - 1) / splits;
     return 10 * even < 9 * longest_share || even > longest_share ? even : longest_share;
@@ -619,7 +621,7 @@ __global__ void __launch_bounds__(AMT_THREADS) attention_decode_tma_kernel(const
     int k_begin, k_end;
     bool idle;
     if (a.cluster_merge) {
-        const int tile0 = lo / AM_TILE, share = decode_share(pos / AM_TILE + 1 - tile0, a.max_splits, a.split / AM_TILE);
+        const int tile0 = lo / AM_TILE, share = decode_share(pos / AM_TILE + 1 - tile0, a.max_splits, a.longest_share);
         k_begin = (tile0 + split * share) * AM_TILE;
         k_end = min(k_begin + share * AM_TILE, pos + 1);
         idle = k_begin >= k_end;                 // the merge skips it
@@ -1148,6 +1150,7 @@ extern "C" int ce_attention_decode_bf16_sink(const void* q, const void* k_pool, 
         }
         a.split = best_m * AM_SPLIT;
         a.max_splits = (max_splits + best_m - 1) / best_m;
+        a.longest_share = pairs * a.max_splits <= slots ? a.split / AM_TILE : 0;
     }
     max_splits = a.max_splits;
     // A merge kernel combines the splits.  CE_ATTN_FUSED_MERGE=1 lets the last block of a (sequence,

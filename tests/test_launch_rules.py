@@ -169,7 +169,7 @@ def test_decode_attention_of_more_clusters_than_the_chip_holds_stands_alone(link
 
 # tiles of a sequence, blocks, tiles a block of the longest context (33 tiles in four blocks: 10, 10, 10, 3, not 9, 9, 9, 6)
 @pytest.mark.parametrize("tiles,blocks,longest,share", [(33, 4, 10, 10), (36, 4, 10, 10), (37, 4, 10, 10), (40, 4, 10, 10), (32, 4, 10, 8), (1, 4, 10, 1),
-                                                        (141, 3, 54, 47), (144, 3, 54, 48), (145, 3, 54, 54), (8, 8, 1, 1), (9, 8, 2, 2), (8, 8, 2, 1), (41, 4, 10, 11)])
+                                                        (141, 3, 54, 47), (144, 3, 54, 48), (145, 3, 54, 54), (8, 8, 1, 1), (9, 8, 2, 2), (8, 8, 2, 1), (41, 4, 10, 11), (33, 4, 0, 9), (1, 3, 0, 1)])
 def test_a_sequences_tiles_are_dealt_evenly_unless_it_is_about_the_longest(linked, tiles, blocks, longest, share):
     assert Chip(linked, {}).lib.ce_attention_decode_share(tiles, blocks, longest) == share
     assert share * blocks >= tiles                                   # nothing is left out
